@@ -44,8 +44,8 @@ __global__ void __launch_bounds__(64) dec_prologue_kernel(FrodoBatch b) {
   else fdev::ct_absorb_inst(inst_of(b, i, OP_DEC));
 }
 
-// Several lanes per state (msponge.cuh; NS = 5: five lanes, six instances per warp; NS = 1:
-// a warp per instance), one warp per block.  STAGE selects the stage body: 0 keypair
+// Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 10: ten lanes, three
+// instances per warp; NS = 2: a pair, sixteen), one warp per block.  STAGE selects the stage body: 0 keypair
 // prologue, 1 H(pk), 2 encaps prologue, 3 encaps final hash, 4 decaps final hash; the
 // decaps prologue below has its own kernel.
 template <int STAGE, int NS>
@@ -147,9 +147,12 @@ __global__ void __launch_bounds__(256, 2) kp_as_tc_kernel(FrodoBatch b) {
 
 inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
-// Lanes per state of a thread-level sponge stage: a warp per state up to warp_max, five lanes
-// up to five_max (frodo_warp_max / frodo_five_max for the prologues, frodo_ss_warp_max /
-// frodo_ss_five_max for the hashes), else one (false: the caller launches that).
+// Lanes per state of a thread-level sponge stage: a warp per state up to warp_max, ten lanes up
+// to five_max (frodo_warp_max / frodo_five_max for the prologues, frodo_ss_warp_max /
+// frodo_ss_five_max for the hashes; the knobs' names are from a layout of five), a pair up to
+// kPairMax (a warp of pairs per SM sub-partition: final hashes at 8,192 0.39 ms against 0.55 on one
+// lane), else one (false: the caller launches that).
+constexpr int kPairMax = 148 * 4 * 16;
 template <int STAGE>
 bool launch_multi(const FrodoBatch &b, int warp_max, int five_max, cudaStream_t st) {
   if (b.n <= warp_max) {
@@ -157,7 +160,11 @@ bool launch_multi(const FrodoBatch &b, int warp_max, int five_max, cudaStream_t 
     return true;
   }
   if (b.n <= five_max) {
-    stage_multi_kernel<STAGE, 5><<<blocks_for(b.n, 6), 32, 0, st>>>(b);
+    stage_multi_kernel<STAGE, 10><<<blocks_for(b.n, 3), 32, 0, st>>>(b);
+    return true;
+  }
+  if (b.n <= kPairMax) {
+    stage_multi_kernel<STAGE, 2><<<blocks_for(b.n, 16), 32, 0, st>>>(b);
     return true;
   }
   return false;
@@ -246,7 +253,7 @@ __global__ void __launch_bounds__(32) pk_digest_kernel(const uint8_t *pk, uint8_
   msp::zero<S>(a);
   const int pos = msp::absorb_aligned<S, 136>(a, s, 0, pk, PK, true);
   msp::absorb_finish<S, 136>(a, s, pos, 0x1Fu);
-  msp::store<S>(a, s, out, 3, true);
+  msp::store<S, 3>(a, s, out, true);
 }
 
 template <class G, int NST>
@@ -331,7 +338,8 @@ cudaError_t frodo_dec(const FrodoBatch &b, int form, cudaStream_t st) {
   dec_w_kernel<<<b.n, 256, fdev::DEC_W_SMEM, st>>>(b);
   mark(b, st);
   if (b.n <= tuning().frodo_warp_max) dec_prologue_multi_kernel<1><<<b.n, 64, 0, st>>>(b);
-  else if (b.n <= tuning().frodo_five_max) dec_prologue_multi_kernel<5><<<blocks_for(b.n, 6), 64, 0, st>>>(b);
+  else if (b.n <= tuning().frodo_five_max) dec_prologue_multi_kernel<10><<<blocks_for(b.n, 3), 64, 0, st>>>(b);
+  else if (b.n <= kPairMax) dec_prologue_multi_kernel<2><<<blocks_for(b.n, 16), 64, 0, st>>>(b);
   else dec_prologue_kernel<<<blocks_for(b.n, 32), 64, 0, st>>>(b);
   mark(b, st);
   cudaError_t e = launch_sa<OP_DEC>(b, form, st);

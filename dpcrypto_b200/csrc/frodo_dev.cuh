@@ -280,64 +280,90 @@ __device__ __forceinline__ void ss_inst(const Inst &v) {
 
 // ---------------------------------------------------------------- several lanes per state
 // The thread-level stages above with each sponge spread over several lanes (msponge.cuh:
-// S = msp::Multi<5>, five lanes per state, or msp::Multi<1>, a warp per state); they write
-// the same bytes.  live = false keeps a state without an instance in step (its reads stay
+// S = msp::Multi<1>, a warp per state, msp::Multi<10>, ten lanes, or msp::Multi<2>, a pair); they
+// write the same bytes.  live = false keeps a state without an instance in step (its reads stay
 // in bounds, its writes are skipped).
-
-__device__ __forceinline__ uint64_t u64_of(uint2 v) { return ((uint64_t)v.y << 32) | v.x; }
-__device__ __forceinline__ uint2 uint2_of(uint64_t v) { return make_uint2((uint32_t)v, (uint32_t)(v >> 32)); }
 
 // dom || seed (25 bytes) absorbed and finished, the 24-byte seed in lanes 0..2 of g:
 // message lane j = (seed lane j-1 >> 56) | (seed lane j << 8), lane 0 with dom.
 template <class S>
-__device__ __forceinline__ void seed_stream_init_multi(uint2 (&a)[S::NS], const S &s, uint32_t dom,
-                                                       const uint2 (&g)[S::NS]) {
-  const uint64_t x0 = u64_of(s.template get<0>(g)), x1 = u64_of(s.template get<1>(g)),
-                 x2 = u64_of(s.template get<2>(g));
+__device__ __forceinline__ void seed_stream_init_multi(typename S::W (&a)[S::NS], const S &s, uint32_t dom,
+                                                       const typename S::W (&g)[S::NS]) {
+  using W = typename S::W;
+  const W x0 = s.template get<0>(g), x1 = s.template get<1>(g), x2 = s.template get<2>(g), z = msp::none<W>();
+  W l0 = S::shl8(z, x0);
+  msp::fold(l0, s.in(s.part(make_uint2(dom, 0u))));
   msp::zero<S>(a);
-#pragma unroll
-  for (int y = 0; y < S::NS; y++) {
-    const int q = s.lane(y);
-    const uint64_t l = q == 0 ? (uint64_t)dom | (x0 << 8)
-                     : q == 1 ? (x0 >> 56) | (x1 << 8)
-                     : q == 2 ? (x1 >> 56) | (x2 << 8)
-                     : q == 3 ? (x2 >> 56)
-                              : 0ull;
-    a[y] = uint2_of(l);
-  }
+  msp::xor_lane<S, 0>(a, s, l0);
+  msp::xor_lane<S, 1>(a, s, S::shl8(x0, x1));
+  msp::xor_lane<S, 2>(a, s, S::shl8(x1, x2));
+  msp::xor_lane<S, 3>(a, s, S::shl8(x2, z));
   msp::absorb_finish<S, 136>(a, s, 25, 0x1Fu);
+}
+
+// One word of two values, as sample_lane's of four.
+__device__ __forceinline__ uint32_t sample_lane(uint32_t w) {
+  const FmaConsts k = fma_consts();
+  return sample16_fma(w, k) | (sample16_fma(w >> 16, k) << 16);
+}
+
+// a where the mask is ones, else b.
+__device__ __forceinline__ uint32_t select_words(uint32_t m, uint32_t a, uint32_t b) { return (a & m) | (b & ~m); }
+__device__ __forceinline__ uint2 select_words(uint32_t m, uint2 a, uint2 b) {
+  return make_uint2(select_words(m, a.x, b.x), select_words(m, a.y, b.y));
 }
 
 // sample_stream on several lanes: each thread samples and stores the rate lanes it owns.
 template <class S>
-__device__ __forceinline__ void sample_stream_multi(uint2 (&a)[S::NS], const S &s, uint16_t *dst, int words,
+__device__ __forceinline__ void sample_stream_multi(typename S::W (&a)[S::NS], const S &s, uint16_t *dst, int words,
                                                     uint8_t *dst_le, int le_words, bool live) {
   const int nblk = (words + 67) / 68;
   for (int blk = 0; blk < nblk; blk++) {
     if (blk) s.perm(a);
+    typename S::W r[S::NS];
 #pragma unroll
-    for (int y = 0; y < S::NS; y++) {
-      const int q = s.lane(y), w = blk * 68 + 4 * q;
-      if (q < 17 && w < words && live && s.writer()) {
-        const uint2 v = sample_lane(a[y]);
-        *reinterpret_cast<uint2 *>(dst + w) = v;
-        if (dst_le && w < le_words) *reinterpret_cast<uint2 *>(dst_le + 2 * w) = v;
+    for (int y = 0; y < S::NS; y++)
+      if (S::least(y) < 17) r[y] = sample_lane(s.out(a[y]));
+#pragma unroll
+    for (int y = 0; y < S::NS; y++)
+      if (S::least(y) < 17) msp::pin(r[y]);
+    if (live && s.writer()) {
+#pragma unroll
+      for (int y = 0; y < S::NS; y++) {
+        if (S::least(y) >= 17) continue;
+        const int q = s.lane(y), w = blk * 68 + 4 * q;
+        if (q < 17 && w < words) {
+          s.store(reinterpret_cast<uint8_t *>(dst + w), r[y]);
+          if (dst_le && w < le_words) s.store(dst_le + 2 * w, r[y]);
+        }
       }
     }
   }
 }
 
+// The state as lanes 0..24 in this instance's scratch.
+template <class S>
+__device__ __forceinline__ void save_state_multi(const typename S::W (&a)[S::NS], const S &s, uint2 *hs, bool live) {
+#pragma unroll
+  for (int y = 0; y < S::NS; y++) {
+    const typename S::W w = s.out(a[y]);
+    if (live && s.writer()) s.store(reinterpret_cast<uint8_t *>(hs + s.lane(y)), w);
+  }
+}
+
 template <class S>
 __device__ __forceinline__ void kp_prologue_multi(const Inst &v, const S &s, bool live) {
-  uint2 a[S::NS], g[S::NS];
+  typename S::W a[S::NS], g[S::NS];
   // seedA = SHAKE256(z, 16)
   msp::zero<S>(a);
   msp::absorb_aligned<S, 136>(a, s, 0, v.coins + 48, 16, live);
   msp::absorb_finish<S, 136>(a, s, 16, 0x1Fu);
-  msp::store<S>(a, s, v.pk, 2, live);
-  msp::store<S>(a, s, v.sk + LENS, 2, live);
-  const int q = s.lane(0);
-  if (live && s.writer() && q < 3) *reinterpret_cast<uint2 *>(v.sk + 8 * q) = ld_lane(v.coins + 8 * q);
+  msp::store<S, 2>(a, s, v.pk, live);
+  msp::store<S, 2>(a, s, v.sk + LENS, live);
+#pragma unroll
+  for (int y = 0; y < S::NS; y++)
+    if (S::least(y) < 3 && live && s.writer() && s.lane(y) < 3)
+      s.store(v.sk + 8 * s.lane(y), s.load(v.coins + 8 * s.lane(y)));
   // S^T || E = sample(SHAKE256(0x5F || seedSE))
   msp::zero<S>(g);
   msp::absorb_aligned<S, 136>(g, s, 0, v.coins + 24, 24, live);
@@ -347,16 +373,16 @@ __device__ __forceinline__ void kp_prologue_multi(const Inst &v, const S &s, boo
 
 template <class S>
 __device__ __forceinline__ void pk_hash_multi(const Inst &v, const S &s, bool live) {
-  uint2 a[S::NS];
+  typename S::W a[S::NS];
   msp::zero<S>(a);
   const int pos = msp::absorb_aligned<S, 136>(a, s, 0, v.pk, PK, live);
   msp::absorb_finish<S, 136>(a, s, pos, 0x1Fu);
-  msp::store<S>(a, s, v.sk + SK_PKH, 3, live);
+  msp::store<S, 3>(a, s, v.sk + SK_PKH, live);
 }
 
 template <class S, int MODE>
 __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, bool live) {
-  uint2 a[S::NS], g[S::NS];
+  typename S::W a[S::NS], g[S::NS];
   msp::zero<S>(g);
   if (MODE == OP_ENC) {
     if (v.pkh) {  // shared-key batch: H(pk) hashed once
@@ -367,7 +393,7 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, bool l
       msp::absorb_finish<S, 136>(a, s, pos, 0x1Fu);
 #pragma unroll
       for (int y = 0; y < S::NS; y++)
-        if (s.lane(y) < 3) g[y] = a[y];  // pkh = lanes 0..2
+        if (S::least(y) < 3 && s.lane(y) < 3) g[y] = a[y];  // pkh = lanes 0..2
     }
     msp::absorb_aligned<S, 136>(g, s, 24, v.coins, 24, live);
   } else {
@@ -378,8 +404,10 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, bool l
   msp::absorb_finish<S, 136>(g, s, 48, 0x1Fu);
 #pragma unroll
   for (int y = 0; y < S::NS; y++) {
+    if (S::least(y) >= 6) continue;
     const int q = s.lane(y);
-    if (q >= 3 && q < 6 && live && s.writer()) *reinterpret_cast<uint2 *>(v.kk + 8 * (q - 3)) = g[y];
+    const typename S::W w = s.out(g[y]);
+    if (q >= 3 && q < 6 && live && s.writer()) s.store(v.kk + 8 * (q - 3), w);
   }
   seed_stream_init_multi<S>(a, s, 0x96u, g);
   sample_stream_multi<S>(a, s, v.rw, RW, nullptr, 0, live);
@@ -387,21 +415,20 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, bool l
 
 template <class S>
 __device__ __forceinline__ void ct_absorb_multi(const Inst &v, const S &s, bool live) {
-  uint2 a[S::NS];
+  typename S::W a[S::NS];
   msp::zero<S>(a);
   msp::absorb_aligned<S, 136>(a, s, 0, v.ct, CT_FULL, live);
-#pragma unroll
-  for (int y = 0; y < S::NS; y++)
-    if (live && s.writer()) v.hs[s.lane(y)] = a[y];
+  save_state_multi<S>(a, s, v.hs, live);
 }
 
 template <class S, int MODE>
 __device__ __forceinline__ void ss_multi(const Inst &v, const S &s, bool live) {
-  uint2 a[S::NS];
+  typename S::W a[S::NS];
   int pos;
   if (MODE == OP_DEC) {
 #pragma unroll
-    for (int y = 0; y < S::NS; y++) a[y] = live ? v.hs[s.lane(y)] : make_uint2(0u, 0u);
+    for (int y = 0; y < S::NS; y++)
+      a[y] = s.in(live ? s.load(reinterpret_cast<const uint8_t *>(v.hs + s.lane(y))) : msp::none<typename S::W>());
     pos = msp::absorb_aligned<S, 136>(a, s, 0, v.ct + CT_FULL, CT - CT_FULL, live);
   } else {
     msp::zero<S>(a);
@@ -413,19 +440,17 @@ __device__ __forceinline__ void ss_multi(const Inst &v, const S &s, bool live) {
   const int q0 = pos / 8;
 #pragma unroll
   for (int y = 0; y < S::NS; y++) {
+    if (S::least(y) >= 17) continue;
     const int q = s.lane(y);
+    typename S::W x = msp::none<typename S::W>();
     if (q >= q0 && q < q0 + 3 && live) {
-      uint2 x = ld_lane(v.kk + 8 * (q - q0));
-      if (MODE == OP_DEC) {
-        const uint2 sv = ld_lane(v.sk + 8 * (q - q0));
-        x = make_uint2((x.x & ~m) | (sv.x & m), (x.y & ~m) | (sv.y & m));
-      }
-      a[y].x ^= x.x;
-      a[y].y ^= x.y;
+      x = s.load(v.kk + 8 * (q - q0));
+      if (MODE == OP_DEC) x = select_words(m, s.load(v.sk + 8 * (q - q0)), x);
     }
+    msp::fold(a[y], s.in(x));
   }
   msp::absorb_finish<S, 136>(a, s, pos + 24, 0x1Fu);
-  msp::store<S>(a, s, v.ss, 3, live);
+  msp::store<S, 3>(a, s, v.ss, live);
 }
 
 // ---------------------------------------------------------------- CTA-level stages (256 threads)

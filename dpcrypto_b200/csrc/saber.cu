@@ -12,25 +12,16 @@ using sdev::inst_of;
 using sdev::PL;
 using sdev::Scr;
 
-// One or two lanes per state: 32 instances per block.  Warp 0 = hash chain + GenSecret XOF
-// (a thread per instance); GenMatrix XOF on warp 1 (a thread per instance, PAIR = false,
-// blockDim 64) or on warps 1-2 (a lane pair per instance, PAIR = true, blockDim 96).  Pairs shorten the longest chain
-// while the batch leaves SM sub-partitions idle, and cost more issue slots per state once
-// it does not (tuning knob saber_pair_max).
-template <int L, int OP, bool PAIR>
-__global__ void __launch_bounds__(96) prologue_kernel(SaberBatch b) {
-  if (!PAIR || threadIdx.x < 32) {
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
-    if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), threadIdx.x >> 5);
-    return;
-  }
-  const int t = threadIdx.x - 32, i = blockIdx.x * 32 + (t >> 1);
-  const bool live = i < b.n;
-  sdev::matrix_pair<L, OP>(inst_of<L>(b, live ? i : b.n - 1, OP), t & 1, live);
+// One lane per state: 32 instances per block; warp 0 the hash chain and GenSecret, warp 1
+// GenMatrix.
+template <int L, int OP>
+__global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b) {
+  const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+  if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), threadIdx.x >> 5);
 }
 
-// Several lanes per state (msponge.cuh; NS = 5: five lanes, six instances per warp; NS = 1:
-// a warp per instance).  Two warps per block: warp 0 the hash chain and GenSecret, warp 1
+// Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 10: ten lanes, three
+// instances per warp; NS = 2: a pair, sixteen).  Two warps per block: warp 0 the hash chain and GenSecret, warp 1
 // GenMatrix, for the same instances.
 template <int L, int OP, int NS>
 __global__ void __launch_bounds__(64) prologue_multi_kernel(SaberBatch b) {
@@ -50,23 +41,15 @@ void launch_prologue_multi(const SaberBatch &b, cudaStream_t st) {
 }
 
 // Lanes per state of the prologue's sponges for a batch of n: a warp per state up to
-// saber_warp_max, five lanes up to saber_five_max, a pair (GenMatrix only) up to
-// saber_pair_max, else one.
+// saber_warp_max, ten lanes up to saber_five_max (the knob's name is from a layout of five), a
+// pair up to saber_pair_max, else one.
 template <int L, int OP>
 void launch_prologue(const SaberBatch &b, cudaStream_t st) {
   const int pb = (b.n + 31) / 32;
   if (b.n <= tuning().saber_warp_max) launch_prologue_multi<L, OP, 1>(b, st);
-  else if (b.n <= tuning().saber_five_max) launch_prologue_multi<L, OP, 5>(b, st);
-  else if (b.n <= tuning().saber_pair_max) prologue_kernel<L, OP, true><<<pb, 96, 0, st>>>(b);
-  else prologue_kernel<L, OP, false><<<pb, 64, 0, st>>>(b);
-}
-
-// Encaps finish on lane pairs, 64 threads = 32 instances.
-template <int L>
-__global__ void __launch_bounds__(64) finish_enc_pair_kernel(SaberBatch b) {
-  const int t = blockIdx.x * 64 + threadIdx.x, i = t >> 1;
-  const bool live = i < b.n;
-  sdev::finish_enc_pair<L>(inst_of<L>(b, live ? i : b.n - 1, OP_ENC), t & 1, live);
+  else if (b.n <= tuning().saber_five_max) launch_prologue_multi<L, OP, 10>(b, st);
+  else if (b.n <= tuning().saber_pair_max) launch_prologue_multi<L, OP, 2>(b, st);
+  else prologue_kernel<L, OP><<<pb, 64, 0, st>>>(b);
 }
 
 // Encaps / keypair finish on several lanes per state, one warp per block.
@@ -82,8 +65,8 @@ __global__ void __launch_bounds__(32) finish_multi_kernel(SaberBatch b) {
   else sdev::finish_kp_multi<S, L>(v, s, live);
 }
 
-// The finish on a warp per state or five lanes per state when n is within the thresholds;
-// false otherwise.
+// The finish on a warp, ten lanes or a pair per state when n is within the thresholds; false
+// otherwise.
 template <int L, int OP>
 bool launch_finish_multi(const SaberBatch &b, cudaStream_t st) {
   if (b.n <= tuning().saber_finish_warp_max) {
@@ -91,7 +74,11 @@ bool launch_finish_multi(const SaberBatch &b, cudaStream_t st) {
     return true;
   }
   if (b.n <= tuning().saber_finish_five_max) {
-    finish_multi_kernel<L, OP, 5><<<(b.n + 5) / 6, 32, 0, st>>>(b);
+    finish_multi_kernel<L, OP, 10><<<(b.n + 2) / 3, 32, 0, st>>>(b);
+    return true;
+  }
+  if (b.n / 2 <= tuning().saber_pair_max) {  // one sponge per instance, the prologue has two
+    finish_multi_kernel<L, OP, 2><<<(b.n + 15) / 16, 32, 0, st>>>(b);
     return true;
   }
   return false;
@@ -253,10 +240,7 @@ cudaError_t run(const SaberBatch &b, int op, int form, cudaStream_t st) {
       mark(b, st);
       if ((e = launch_product<L, sdev::PM_ENC>(b, form, st)) != cudaSuccess) return e;
       mark(b, st);
-      if (!launch_finish_multi<L, OP_ENC>(b, st)) {
-        if (b.n <= tuning().saber_pair_max) finish_enc_pair_kernel<L><<<(b.n + 31) / 32, 64, 0, st>>>(b);
-        else finish_kernel<L, OP_ENC><<<fb, tb, 0, st>>>(b);
-      }
+      if (!launch_finish_multi<L, OP_ENC>(b, st)) finish_kernel<L, OP_ENC><<<fb, tb, 0, st>>>(b);
       break;
     default:
       if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st)) != cudaSuccess) return e;

@@ -30,7 +30,6 @@
 #pragma once
 #include "common.cuh"
 #include "keccak.cuh"
-#include "keccak_pair.cuh"
 #include "msponge.cuh"
 #include "tc.cuh"
 
@@ -219,82 +218,23 @@ __device__ __forceinline__ void prologue_inst(const Inst &v, int role) {
   }
 }
 
-// GenMatrix (prologue role 1) on a lane pair (p = lane parity): its 10 / 23 / 40 permutations are
-// the longest chain of the prologue.  live = false keeps a padding pair of a partial warp in
-// step (its reads are valid, its writes are skipped).
-template <int L, int OP>
-__device__ __forceinline__ void matrix_pair(const Inst &v, int p, bool live) {
-  using P = SP<L>;
-  using S = Scr<L>;
-  uint32_t a[25];
-  kpair::zero(a);
-  if (OP == OP_KEYPAIR) {
-    // seed_A = SHAKE128(coins[0:32], 32), published in pk.
-#pragma unroll
-    for (int q = 0; q < 4; q++) a[q] = kpair::to_slice(ld_lane(v.coins + 8 * q), p);
-    kpair::absorb_finish<168>(a, 32, 0x1Fu, p);
-    uint32_t seed[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      seed[q] = a[q];
-      const uint32_t h = kpair::from_slice(a[q], p);
-      if (live) *reinterpret_cast<uint32_t *>(v.pk + P::POLYVECCOMP + 8 * q + 4 * p) = h;
-    }
-    kpair::zero(a);
-#pragma unroll
-    for (int q = 0; q < 4; q++) a[q] = seed[q];
-  } else {
-    const uint8_t *src = OP == OP_ENC ? v.pk + P::POLYVECCOMP : v.sk + P::POLYVEC + P::POLYVECCOMP;
-#pragma unroll
-    for (int q = 0; q < 4; q++) a[q] = kpair::to_slice(ld_lane(src + 8 * q), p);
-  }
-  kpair::absorb_finish<168>(a, 32, 0x1Fu, p);
-  kpair::squeeze<168>(a, v.scr + S::ARAW, P::ARAW, p, live);
-}
-
-// Encaps finish on a lane pair: k = SHA3-256(kr[0:32] || SHA3-256(c)), the same bytes as
-// finish_inst<L, OP_ENC>; 10 dependent permutations at l = 3.
-template <int L>
-__device__ __forceinline__ void finish_enc_pair(const Inst &v, int p, bool live) {
-  using P = SP<L>;
-  using S = Scr<L>;
-  uint32_t a[25], hc[4];
-  kpair::zero(a);
-  const int pos = kpair::absorb_aligned<136>(a, 0, v.ct, P::CT, p);
-  kpair::absorb_finish<136>(a, pos, 0x06u, p);
-#pragma unroll
-  for (int q = 0; q < 4; q++) hc[q] = a[q];
-  kpair::zero(a);
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    a[q] = kpair::to_slice(ld_lane(v.scr + S::KR + 8 * q), p);
-    a[4 + q] = hc[q];
-  }
-  kpair::absorb_finish<136>(a, 64, 0x06u, p);
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const uint32_t h = kpair::from_slice(a[q], p);
-    if (live) *reinterpret_cast<uint32_t *>(v.ss + 8 * q + 4 * p) = h;
-  }
-}
-
 // ---------------------------------------------------------------- several lanes per state
 // The same prologue roles and encaps / keypair finish with each sponge spread over several
-// lanes (msponge.cuh: S = msp::Multi<5>, five lanes per state, or msp::Multi<1>, a warp per
-// state): the bytes written are those of prologue_inst / finish_inst.  live = false keeps a
+// lanes (msponge.cuh: S = msp::Multi<1>, a warp per state, msp::Multi<10>, ten lanes, or
+// msp::Multi<2>, a pair): the bytes written are those of prologue_inst / finish_inst.  live = false keeps a
 // state without an instance in step (reads stay in bounds, writes are skipped).
 template <class S, int L, int OP>
 __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int role, bool live) {
   using P = SP<L>;
   using Q = Scr<L>;
   uint8_t *scr = v.scr;
-  uint2 a[S::NS];
+  typename S::W a[S::NS];
   msp::zero<S>(a);
   if (role == 1) {  // GenMatrix
     if (OP == OP_KEYPAIR) {  // seed_A = SHAKE128(coins[0:32], 32), published in pk
       msp::absorb_aligned<S, 168>(a, s, 0, v.coins, 32, live);
       msp::absorb_finish<S, 168>(a, s, 32, 0x1Fu);
-      msp::store<S>(a, s, v.pk + P::POLYVECCOMP, 4, live);
+      msp::store<S, 4>(a, s, v.pk + P::POLYVECCOMP, live);
       msp::keep<S>(a, s, 4);
     } else {
       const uint8_t *src = OP == OP_ENC ? v.pk + P::POLYVECCOMP : v.sk + P::POLYVEC + P::POLYVECCOMP;
@@ -307,13 +247,13 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int ro
   if (OP == OP_KEYPAIR) {
     msp::absorb_aligned<S, 168>(a, s, 0, v.coins + 32, 32, live);
   } else {
-    uint2 kr[S::NS];
+    typename S::W kr[S::NS];
     msp::zero<S>(kr);
     if (OP == OP_ENC) {
       // m = SHA3-256(coins), H(pk), kr = SHA3-512(m || H(pk))  (cuda_kernel.cu:68-70)
       msp::absorb_aligned<S, 136>(kr, s, 0, v.coins, 32, live);
       msp::absorb_finish<S, 136>(kr, s, 32, 0x06u);
-      msp::store<S>(kr, s, scr + Q::MTXT, 4, live);
+      msp::store<S, 4>(kr, s, scr + Q::MTXT, live);
       msp::keep<S>(kr, s, 4);  // lanes 0..3 = m
       const int pos = msp::absorb_aligned<S, 136>(a, s, 0, v.pk, P::PK, live);
       msp::absorb_finish<S, 136>(a, s, pos, 0x06u);
@@ -324,7 +264,7 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int ro
       msp::absorb_aligned<S, 72>(kr, s, pos, v.sk + P::SK - 64, 32, live);
     }
     msp::absorb_finish<S, 72>(kr, s, 64, 0x06u);
-    msp::store<S>(kr, s, scr + Q::KR, 8, live);
+    msp::store<S, 8>(kr, s, scr + Q::KR, live);
     // GenSecret seed = kr[32:64] = lanes 4..7 -> lanes 0..3
     msp::zero<S>(a);
     msp::xor_lane<S, 0>(a, s, s.template get<4>(kr));
@@ -338,7 +278,7 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int ro
     msp::zero<S>(a);
     const int pos = msp::absorb_aligned<S, 136>(a, s, 0, v.ct, P::CT, live);
     msp::absorb_finish<S, 136>(a, s, pos, 0x06u);
-    msp::store<S>(a, s, scr + Q::HC, 4, live);
+    msp::store<S, 4>(a, s, scr + Q::HC, live);
   }
 }
 
@@ -347,7 +287,7 @@ template <class S, int L>
 __device__ __forceinline__ void finish_enc_multi(const Inst &v, const S &s, bool live) {
   using P = SP<L>;
   using Q = Scr<L>;
-  uint2 h[S::NS], a[S::NS];
+  typename S::W h[S::NS], a[S::NS];
   msp::zero<S>(h);
   const int pos = msp::absorb_aligned<S, 136>(h, s, 0, v.ct, P::CT, live);
   msp::absorb_finish<S, 136>(h, s, pos, 0x06u);
@@ -355,26 +295,28 @@ __device__ __forceinline__ void finish_enc_multi(const Inst &v, const S &s, bool
   msp::absorb_aligned<S, 136>(a, s, 0, v.scr + Q::KR, 32, live);
   msp::move4<S, 4>(a, h, s);
   msp::absorb_finish<S, 136>(a, s, 64, 0x06u);
-  msp::store<S>(a, s, v.ss, 4, live);
+  msp::store<S, 4>(a, s, v.ss, live);
 }
 
 // Keypair finish: sk = s || pk || H(pk) || z (the secret part was written by the product).
 template <class S, int L>
 __device__ __forceinline__ void finish_kp_multi(const Inst &v, const S &s, bool live) {
   using P = SP<L>;
-  if (live && s.writer()) {
-    const int t = s.lane(0) % 5;  // five threads share the copy (a warp per state: lanes 0..4)
-    if (s.lane(0) < 5)
-      for (int off = 8 * t; off < P::PK; off += 40)
-        *reinterpret_cast<uint2 *>(v.sk + P::POLYVEC + off) = ld_lane(v.pk + off);
+  if (live && s.writer()) {  // pk, words t, t + T, ... on thread t of the state's T
+    constexpr int T = 32 / S::STATES_PER_WARP < 25 ? 32 / S::STATES_PER_WARP : 25;
+    const int t = (int)(threadIdx.x & 31) - T * s.state();
+    for (int off = 8 * t; off < P::PK; off += 8 * T)
+      *reinterpret_cast<uint2 *>(v.sk + P::POLYVEC + off) = ld_lane(v.pk + off);
   }
-  uint2 a[S::NS];
+  typename S::W a[S::NS];
   msp::zero<S>(a);
   const int pos = msp::absorb_aligned<S, 136>(a, s, 0, v.pk, P::PK, live);
   msp::absorb_finish<S, 136>(a, s, pos, 0x06u);
-  msp::store<S>(a, s, v.sk + P::SK - 64, 4, live);
-  const int q = s.lane(0);
-  if (live && s.writer() && q < 4) *reinterpret_cast<uint2 *>(v.sk + P::SK - 32 + 8 * q) = ld_lane(v.coins + 64 + 8 * q);
+  msp::store<S, 4>(a, s, v.sk + P::SK - 64, live);
+#pragma unroll
+  for (int y = 0; y < S::NS; y++)
+    if (S::least(y) < 4 && live && s.writer() && s.lane(y) < 4)
+      s.store(v.sk + P::SK - 32 + 8 * s.lane(y), s.load(v.coins + 64 + 8 * s.lane(y)));
 }
 
 // ---------------------------------------------------------------- finish
