@@ -133,6 +133,8 @@ namespace {
 
 constexpr size_t kPipeChunkMin = 256;  // smallest chunk of a host-mode pipeline
 constexpr size_t kDefaultBudget = 8ull << 30;
+// The error word and, 256 bytes apart, one work queue (two words) per pipeline slot.
+constexpr size_t kQueueStride = 64, kErrBytes = (1 + kPipeChunks) * kQueueStride * 4;
 
 struct Carver {
   uint8_t *base;
@@ -219,7 +221,14 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
       edge = e;
     }
   }
-  const size_t per_pipe = (arena_need(scheme, op, chunk, !dev) + kAlign - 1) & ~(kAlign - 1);
+  const size_t base = arena_need(scheme, op, chunk, !dev);
+  // FrodoKEM on the tensor cores: operand tiles for A generated ahead, as far as the budget
+  // leaves room (none at all is a valid answer).
+  const bool frodo_tc = scheme <= DPKEM_FRODO976AES && form == DPKEM_FORM_TC;
+  size_t tile_cap = 0;
+  if (frodo_tc && c->budget / npipe > base + kAlign)
+    tile_cap = (size_t)frodo_ahead_count((int)chunk, (c->budget / npipe - base - kAlign) / frodo_ahead_bytes());
+  const size_t per_pipe = up(base + tile_cap * frodo_ahead_bytes());
   int rc = ensure_arena(c, per_pipe * npipe);
   if (rc) return rc;
   cudaError_t e = cudaStreamWaitEvent(st, c->last, 0);
@@ -289,6 +298,11 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
       fb.n = (int)m;
       fb.aes = scheme == DPKEM_FRODO976AES;
       fb.err = c->d_err;
+      if (tile_cap) {
+        fb.atile = c->arena + (size_t)j * per_pipe + base;
+        fb.ahead = frodo_ahead_count((int)m, tile_cap);
+        fb.queue = c->d_err + (1 + j) * kQueueStride;
+      }
       switch (op) {
         case OP_KEYPAIR:
           fb.coins = d_in0; fb.pk = d_out0; fb.sk = d_out1;
@@ -471,7 +485,7 @@ int dpkem_ctx_create(dpkem_ctx **out, int device, size_t hbm_budget_bytes) {
   }
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->last, cudaEventDisableTiming) != cudaSuccess ||
-      cudaMalloc(&c->d_err, 4) != cudaSuccess || cudaMemset(c->d_err, 0, 4) != cudaSuccess) {
+      cudaMalloc(&c->d_err, kErrBytes) != cudaSuccess || cudaMemset(c->d_err, 0, kErrBytes) != cudaSuccess) {
     cudaGetLastError();
     dpkem_ctx_destroy(c);
     return set_status(DPKEM_ECUDA);

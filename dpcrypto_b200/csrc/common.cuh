@@ -99,6 +99,11 @@ struct FrodoBatch {
   // ([A | B] limb tiles, fgemm::AB_BYTES; S' tiles, fgemm::s_bytes(n)); null: per-instance path.
   uint8_t *abt;
   uint8_t *stile;
+  // Tensor-core form with a key per instance: A of the first `ahead` instances is generated
+  // beside the prologue into these operand tiles (frodo_ahead.cuh); null: none.
+  uint8_t *atile;
+  int ahead;
+  uint32_t *queue;  // two zeroed words of the front kernel's row queue
 };
 
 struct SaberBatch {
@@ -128,6 +133,10 @@ cudaError_t frodo_dec(const FrodoBatch &b, int form, cudaStream_t st);
 cudaError_t frodo_expand_a(int aes, const uint8_t *pk, uint16_t *amat, cudaStream_t st);
 // Scratch of the shared-key tensor-core GEMM: [A | B] operand tiles, S' tiles for n instances.
 size_t frodo_gemm_ab_bytes();
+// Instances of a batch of n whose A is generated ahead, given scratch for at most `cap` of
+// them, and that scratch per instance.
+int frodo_ahead_count(int n, size_t cap);
+size_t frodo_ahead_bytes();
 size_t frodo_gemm_s_bytes(size_t n);
 cudaError_t frodo_pk_digest(const uint8_t *pk, uint8_t *out, cudaStream_t st);
 

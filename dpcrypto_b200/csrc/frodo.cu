@@ -1,7 +1,10 @@
 // FrodoKEM-976 (SHAKE and AES variants) batched keypair / encaps / decaps: one launch per
 // stage over n instances.  The stage bodies live in frodo_dev.cuh (shared with the persistent
 // mixed-batch kernel); these wrappers only map blockIdx/threadIdx to instances.
+#include <algorithm>
+
 #include "frodo_dev.cuh"
+#include "frodo_ahead.cuh"
 #include "frodo_gemm.cuh"
 
 namespace dpkem {
@@ -280,6 +283,101 @@ inline void mark(const FrodoBatch &b, cudaStream_t st) {
   if (b.timer) b.timer->mark(st);
 }
 
+// ---- A generated ahead (frodo_ahead.cuh) ----
+
+// Instances [first, n) of a batch (a key per instance).
+FrodoBatch rest_of(const FrodoBatch &b, int first, int op) {
+  FrodoBatch r = b;
+  const size_t i = (size_t)first;
+  r.n = b.n - first;
+  if (b.coins) r.coins = b.coins + i * (op == OP_KEYPAIR ? KP_COINS : ENC_COINS);
+  if (b.pk) r.pk = b.pk + i * PK;
+  if (b.sk) r.sk = b.sk + i * SK;
+  if (b.ct) r.ct = b.ct + i * CT;
+  if (b.ss) r.ss = b.ss + i * SS;
+  r.rw = b.rw + i * RW;
+  r.kk = b.kk + i * LENSE;
+  r.mu = b.mu + i * LENMU;
+  r.fail = b.fail + i;
+  if (b.hs) r.hs = b.hs + i * 25;
+  r.atile = nullptr;
+  r.ahead = 0;
+  return r;
+}
+
+int sm_count() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0, m = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
+    sms = m > 0 ? m : 1;
+  }
+  return sms;
+}
+
+// Chain warps of a front block on ten lanes: four (one per SM sub-partition, 2.05 us per
+// permutation) while the chains outlast the rows, else eight (2.5 us, half the SMs): 2.8 us of the
+// whole chip per instance's rows against the chain's steps.  Measured, n = 128 / 256: encaps 4
+// warps 824 / 1,185 us, 8 warps 902 / 1,164 us; keypair (half the steps) 754 / 1,171 and 701 / 1,120.
+int chain_warps(int ahead, int steps) { return ahead * 28 > steps * 25 ? 8 : 4; }
+
+template <int STAGE, int NS, bool HALVE, class G>
+cudaError_t launch_front_g(const FrodoBatch &b, cudaStream_t st) {
+  cudaError_t e;
+  constexpr int spw = NS == 10 ? 3 : 32;
+  constexpr int steps = STAGE == ahead::F_KEYPAIR ? (HALVE ? 115 : 230) : STAGE == ahead::F_ENC && !HALVE ? 348 : 232;
+  const int warps = blocks_for(b.n, spw), cw = NS == 10 ? chain_warps(b.ahead, steps) : 4, chain = blocks_for(warps, cw);
+  const int absorb = STAGE == ahead::F_DEC ? blocks_for(warps, NS == 10 ? 8 : ahead::kFrontWarps) : 0;
+  const int early = std::max(0, sm_count() - chain - absorb);
+  const int rows = std::min(sm_count(), std::max(1, ahead::WarpRows<G>::tasks(b.ahead)));
+  if ((e = set_smem(ahead::front_kernel<STAGE, NS, HALVE, G>, ahead::kFrontSmem)) != cudaSuccess) return e;
+  ahead::front_kernel<STAGE, NS, HALVE, G>
+      <<<chain + absorb + rows, 32 * ahead::kFrontWarps, ahead::kFrontSmem, st>>>(b, cw, chain, absorb, std::min(early, rows));
+  return cudaGetLastError();
+}
+template <int STAGE, int NS, bool HALVE>
+cudaError_t launch_front_ns(const FrodoBatch &b, cudaStream_t st) {
+  return b.aes ? launch_front_g<STAGE, NS, HALVE, fdev::AesRowsFull>(b, st)
+               : launch_front_g<STAGE, NS, HALVE, fdev::ShakeRows>(b, st);
+}
+// Ten lanes per state up to kFrontTenMax: beyond, the chains' SMs on one lane cost less (a
+// permutation is 135 integer instructions per state there, 160 on ten lanes) than their shorter latency gains,
+// since the rows fill the other SMs meanwhile.  `halve` (encaps, keypair): stop the stream after S',
+// tail_kernel runs the rest.
+constexpr int kFrontTenMax = 4096;
+template <int STAGE>
+cudaError_t launch_front(const FrodoBatch &b, bool halve, cudaStream_t st) {
+  if constexpr (STAGE != ahead::F_DEC)
+    if (halve) return launch_front_ns<STAGE, 10, true>(b, st);
+  if (b.n <= kFrontTenMax) return launch_front_ns<STAGE, 10, false>(b, st);
+  return launch_front_ns<STAGE, 0, false>(b, st);
+}
+
+// Column blocks per product CTA: the whole chip has to be busy with few instances; with many,
+// a CTA per instance part of four blocks reads S' three times instead of twelve.
+template <int MODE>
+cudaError_t launch_product(const FrodoBatch &b, cudaStream_t st) {
+  cudaError_t e;
+  const int nb = b.ahead * 12 <= 592 ? 1 : b.ahead * 6 <= 592 ? 2 : 4;
+  const uint32_t cols = nb <= 2 ? 32 : 64;
+  if ((e = set_smem(ahead::product_kernel<MODE>, ahead::PLayout::total)) != cudaSuccess) return e;
+  ahead::product_kernel<MODE><<<b.ahead * (ahead::BLKS / nb), 256, ahead::PLayout::total, st>>>(b, nb, cols);
+  return cudaGetLastError();
+}
+template <bool RAW>
+cudaError_t launch_product_kp(const FrodoBatch &b, cudaStream_t st) {
+  cudaError_t e;
+  if ((e = set_smem(ahead::product_kp_kernel<RAW>, ahead::KLayout::total)) != cudaSuccess) return e;
+  ahead::product_kp_kernel<RAW><<<b.ahead * ahead::TILES, 256, ahead::KLayout::total, st>>>(b);
+  return cudaGetLastError();
+}
+
+// Whether the batch runs the halved stream and the stepped tail: every instance's products must
+// come raw from product_kernel, and the sponges must be on a warp per state.
+bool halved(const FrodoBatch &b) { return b.ahead == b.n; }
+bool use_ahead(const FrodoBatch &b, int form) { return form == FORM_TC && b.atile && b.ahead > 0 && !b.amat; }
+
 }  // namespace
 
 cudaError_t frodo_expand_a(int aes, const uint8_t *pk, uint16_t *amat, cudaStream_t st) {
@@ -301,9 +399,44 @@ cudaError_t frodo_pk_digest(const uint8_t *pk, uint8_t *out, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+size_t frodo_ahead_bytes() { return ahead::A_BYTES; }
+
+// Batches up to kAheadAll are generated whole: rows are dealt evenly over the SMs, while
+// sa_tc_kernel's two CTAs per SM run in waves of 296 instances (0.88 ms each, 0.5 ms for one
+// instance), and errors and final hash then run in step (tail_kernel).  Above it the A stage runs for the
+// others; an ahead part of 296 .. 591 instances fills the SMs that the prologue leaves free, and
+// leaves whole waves.  Measured ms, encaps: n = 768 all ahead 2.80, 176 ahead 3.45; 1,024 all
+// 3.65, 432 ahead 3.83, none 4.6; 8,192: none 26.99, 200 ahead 26.23, 350 25.83, 496 25.65, 560 25.87.
+constexpr int kAheadAll = 1024;
+
+int frodo_ahead_count(int n, size_t cap) {
+  const int wave = 2 * sm_count(), m = n <= kAheadAll ? n : wave + n % wave;
+  return (int)std::min<size_t>(m, cap);
+}
+
 cudaError_t frodo_keypair(const FrodoBatch &b, int form, cudaStream_t st) {
   if (b.n <= 0) return cudaSuccess;
   const int tb = tuning().thread_block;
+  if (use_ahead(b, form)) {
+    cudaError_t e;
+    const bool half = halved(b);
+    mark(b, st);
+    ahead::kp_seed_kernel<<<blocks_for(b.n, 32), 32, 0, st>>>(b);
+    if ((e = launch_front<ahead::F_KEYPAIR>(b, half, st)) != cudaSuccess) return e;
+    mark(b, st);
+    if ((e = half ? launch_product_kp<true>(b, st) : launch_product_kp<false>(b, st)) != cudaSuccess) return e;
+    if (b.ahead < b.n) {
+      const FrodoBatch r = rest_of(b, b.ahead, OP_KEYPAIR);
+      e = b.aes ? launch_kp_as<fdev::AesRowsFull, 1>(r, form, st) : launch_kp_as<fdev::ShakeRows, fdev::KPT_NST>(r, form, st);
+      if (e != cudaSuccess) return e;
+    }
+    mark(b, st);
+    if (half) ahead::tail_kernel<OP_KEYPAIR><<<blocks_for(b.n, 3), 96, 0, st>>>(b);
+    else if (!launch_multi<1>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st))
+      pk_hash_kernel<OP_KEYPAIR><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
+    mark(b, st);
+    return cudaGetLastError();
+  }
   mark(b, st);
   if (!launch_multi<0>(b, tuning().frodo_warp_max, tuning().frodo_five_max, st))
     kp_prologue_kernel<OP_KEYPAIR><<<blocks_for(b.n, tb), tb, kParkBytes * tb, st>>>(b);
@@ -320,6 +453,21 @@ cudaError_t frodo_keypair(const FrodoBatch &b, int form, cudaStream_t st) {
 cudaError_t frodo_enc(const FrodoBatch &b, int form, cudaStream_t st) {
   if (b.n <= 0) return cudaSuccess;
   const int tb = tuning().thread_block;
+  if (use_ahead(b, form)) {
+    cudaError_t e;
+    const bool half = halved(b);
+    mark(b, st);
+    if ((e = launch_front<ahead::F_ENC>(b, half, st)) != cudaSuccess) return e;
+    mark(b, st);
+    if ((e = half ? launch_product<ahead::PM_RAW>(b, st) : launch_product<ahead::PM_ENC>(b, st)) != cudaSuccess) return e;
+    if (b.ahead < b.n && (e = launch_sa<OP_ENC>(rest_of(b, b.ahead, OP_ENC), form, st)) != cudaSuccess) return e;
+    mark(b, st);
+    if (half) ahead::tail_kernel<OP_ENC><<<blocks_for(b.n, 3), 96, 0, st>>>(b);
+    else if (!launch_multi<3>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st))
+      ss_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
+    mark(b, st);
+    return cudaGetLastError();
+  }
   mark(b, st);
   if (!launch_multi<2>(b, tuning().frodo_warp_max, tuning().frodo_five_max, st)) prologue_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, kParkBytes * tb, st>>>(b);
   mark(b, st);
@@ -337,6 +485,18 @@ cudaError_t frodo_dec(const FrodoBatch &b, int form, cudaStream_t st) {
   mark(b, st);
   dec_w_kernel<<<b.n, 256, fdev::DEC_W_SMEM, st>>>(b);
   mark(b, st);
+  if (use_ahead(b, form)) {
+    cudaError_t e;
+    if ((e = launch_front<ahead::F_DEC>(b, false, st)) != cudaSuccess) return e;
+    mark(b, st);
+    if ((e = launch_product<ahead::PM_DEC>(b, st)) != cudaSuccess) return e;
+    if (b.ahead < b.n && (e = launch_sa<OP_DEC>(rest_of(b, b.ahead, OP_DEC), form, st)) != cudaSuccess) return e;
+    mark(b, st);
+    if (!launch_multi<4>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st))
+      ss_kernel<OP_DEC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
+    mark(b, st);
+    return cudaGetLastError();
+  }
   if (b.n <= tuning().frodo_warp_max) dec_prologue_multi_kernel<1><<<b.n, 64, 0, st>>>(b);
   else if (b.n <= tuning().frodo_five_max) dec_prologue_multi_kernel<10><<<blocks_for(b.n, 3), 64, 0, st>>>(b);
   else if (b.n <= kPairMax) dec_prologue_multi_kernel<2><<<blocks_for(b.n, 16), 64, 0, st>>>(b);
