@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(64) dec_prologue_kernel(FrodoBatch b) {
 // Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 10: ten lanes, three
 // instances per warp; NS = 2: a pair, sixteen), one warp per block.  STAGE selects the stage body: 0 keypair
 // prologue, 1 H(pk), 2 encaps prologue, 3 encaps final hash, 4 decaps final hash; the
-// decaps prologue below has its own kernel.
+// decaps prologue has its own kernels.
 template <int STAGE, int NS>
 __global__ void __launch_bounds__(32) stage_multi_kernel(FrodoBatch b) {
   using S = msp::Multi<NS>;
@@ -65,21 +65,6 @@ __global__ void __launch_bounds__(32) stage_multi_kernel(FrodoBatch b) {
   else if constexpr (STAGE == 2) fdev::prologue_multi<S, OP_ENC>(v, s, live);
   else if constexpr (STAGE == 3) fdev::ss_multi<S, OP_ENC>(v, s, live);
   else fdev::ss_multi<S, OP_DEC>(v, s, live);
-}
-
-// Decaps prologue on several lanes per state: 64 threads, warp 0 the sampling chain, warp 1
-// the ciphertext pre-absorb of the final hash, for the same instances.
-template <int NS>
-__global__ void __launch_bounds__(64) dec_prologue_multi_kernel(FrodoBatch b) {
-  using S = msp::Multi<NS>;
-  __shared__ __align__(16) uint8_t xbuf[2 * (S::SMEM_PER_WARP > 0 ? S::SMEM_PER_WARP : 16)];
-  const int w = threadIdx.x >> 5;
-  const S s(xbuf + w * S::SMEM_PER_WARP);
-  const int g = s.state(), i = blockIdx.x * S::STATES_PER_WARP + g;
-  const bool live = g < S::STATES_PER_WARP && i < b.n;
-  const fdev::Inst v = inst_of(b, live ? i : b.n - 1, OP_DEC);
-  if (w == 0) fdev::prologue_multi<S, OP_DEC>(v, s, live);
-  else fdev::ct_absorb_multi<S>(v, s, live);
 }
 
 template <int MODE>
@@ -150,9 +135,8 @@ __global__ void __launch_bounds__(256, 2) kp_as_tc_kernel(FrodoBatch b) {
 
 inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
-// Lanes per state of a thread-level sponge stage: a warp per state up to warp_max, ten lanes up
-// to five_max (frodo_warp_max / frodo_five_max for the prologues, frodo_ss_warp_max /
-// frodo_ss_five_max for the hashes; the knobs' names are from a layout of five), a pair up to
+// Lanes per state of a hash stage: a warp per state up to warp_max (frodo_ss_warp_max), ten lanes
+// up to five_max (frodo_ss_five_max; the name is from a layout of five), a pair up to
 // kPairMax (a warp of pairs per SM sub-partition: final hashes at 8,192 0.39 ms against 0.55 on one
 // lane), else one (false: the caller launches that).
 constexpr int kPairMax = 148 * 4 * 16;
@@ -279,6 +263,25 @@ cudaError_t launch_kp_as(const FrodoBatch &b, int form, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// The prologue without A's rows: on chain and helper warps up to frodo_warp_max / frodo_five_max
+// (decaps, whose ciphertext hash shares the SMs, up to two thirds of that), encaps and keypair
+// on pairs up to kPairMax; false above.  us, encaps under one key: n = 4,096 780 (five lanes 1,082),
+// 6,000 995, 8,192 on pairs 1,088, on one lane 1,497; decaps: 512 469 (a warp per state 682), 4,096 932
+// (five lanes 1,665), 5,000 1,448 against 1,470 on one lane.
+template <int ROLE>
+bool launch_prologue(const FrodoBatch &b, cudaStream_t st) {
+  const int most = std::max(tuning().frodo_warp_max, tuning().frodo_five_max);
+  if (b.n <= (ROLE == ahead::R_DEC ? most - most / 3 : most)) {
+    const int chain = blocks_for(b.n, 6), absorb = ROLE == ahead::R_DEC ? blocks_for(b.n, 16 * ahead::kAbsorbWarps) : 0;
+    if (ROLE == ahead::R_KEYPAIR) ahead::kp_seed_kernel<<<blocks_for(b.n, 32), 32, 0, st>>>(b);
+    ahead::chains_kernel<ROLE><<<chain + absorb, 128, ahead::chain_smem(2), st>>>(b, chain);
+    return true;
+  }
+  if (ROLE == ahead::R_DEC || b.n > kPairMax) return false;
+  stage_multi_kernel<ROLE == ahead::R_KEYPAIR ? 0 : 2, 2><<<blocks_for(b.n, 16), 32, 0, st>>>(b);
+  return true;
+}
+
 inline void mark(const FrodoBatch &b, cudaStream_t st) {
   if (b.timer) b.timer->mark(st);
 }
@@ -328,7 +331,7 @@ cudaError_t launch_front_g(const FrodoBatch &b, cudaStream_t st) {
   constexpr int spw = NS == 10 ? 3 : 32;
   constexpr int steps = STAGE == ahead::F_KEYPAIR ? (HALVE ? 115 : 230) : STAGE == ahead::F_ENC && !HALVE ? 348 : 232;
   const int warps = blocks_for(b.n, spw), cw = NS == 10 ? chain_warps(b.ahead, steps) : 4, chain = blocks_for(warps, cw);
-  const int absorb = STAGE == ahead::F_DEC ? blocks_for(warps, NS == 10 ? 8 : ahead::kFrontWarps) : 0;
+  const int absorb = STAGE == ahead::F_DEC ? (NS == 10 ? blocks_for(b.n, 16 * ahead::kAbsorbWarps) : blocks_for(warps, ahead::kFrontWarps)) : 0;
   const int early = std::max(0, sm_count() - chain - absorb);
   const int rows = std::min(sm_count(), std::max(1, ahead::WarpRows<G>::tasks(b.ahead)));
   if ((e = set_smem(ahead::front_kernel<STAGE, NS, HALVE, G>, ahead::kFrontSmem)) != cudaSuccess) return e;
@@ -438,7 +441,7 @@ cudaError_t frodo_keypair(const FrodoBatch &b, int form, cudaStream_t st) {
     return cudaGetLastError();
   }
   mark(b, st);
-  if (!launch_multi<0>(b, tuning().frodo_warp_max, tuning().frodo_five_max, st))
+  if (!launch_prologue<ahead::R_KEYPAIR>(b, st))
     kp_prologue_kernel<OP_KEYPAIR><<<blocks_for(b.n, tb), tb, kParkBytes * tb, st>>>(b);
   mark(b, st);
   const cudaError_t e = b.aes ? launch_kp_as<fdev::AesRowsFull, 1>(b, form, st)
@@ -469,7 +472,7 @@ cudaError_t frodo_enc(const FrodoBatch &b, int form, cudaStream_t st) {
     return cudaGetLastError();
   }
   mark(b, st);
-  if (!launch_multi<2>(b, tuning().frodo_warp_max, tuning().frodo_five_max, st)) prologue_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, kParkBytes * tb, st>>>(b);
+  if (!(b.pkh ? launch_prologue<ahead::R_ENC_PKH>(b, st) : launch_prologue<ahead::R_ENC>(b, st))) prologue_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, kParkBytes * tb, st>>>(b);
   mark(b, st);
   cudaError_t e = launch_sa<OP_ENC>(b, form, st);
   if (e != cudaSuccess) return e;
@@ -497,10 +500,7 @@ cudaError_t frodo_dec(const FrodoBatch &b, int form, cudaStream_t st) {
     mark(b, st);
     return cudaGetLastError();
   }
-  if (b.n <= tuning().frodo_warp_max) dec_prologue_multi_kernel<1><<<b.n, 64, 0, st>>>(b);
-  else if (b.n <= tuning().frodo_five_max) dec_prologue_multi_kernel<10><<<blocks_for(b.n, 3), 64, 0, st>>>(b);
-  else if (b.n <= kPairMax) dec_prologue_multi_kernel<2><<<blocks_for(b.n, 16), 64, 0, st>>>(b);
-  else dec_prologue_kernel<<<blocks_for(b.n, 32), 64, 0, st>>>(b);
+  if (!launch_prologue<ahead::R_DEC>(b, st)) dec_prologue_kernel<<<blocks_for(b.n, 32), 64, 0, st>>>(b);
   mark(b, st);
   cudaError_t e = launch_sa<OP_DEC>(b, form, st);
   if (e != cudaSuccess) return e;

@@ -162,25 +162,32 @@ __device__ __forceinline__ void rows_block(const FrodoBatch &b, int block, int b
 // the previous one's output) an idle step, in which the helper forms the message, and an
 // absorbing step from a zero state; then squeezing steps.
 //   encaps   A = 115 (H(pk)), G2, seed          keypair  A = 1 (seed)
-//   decaps   A = 1 (G2), seed                   absorb   A = 115 (ct's full blocks), no squeezing
+//   decaps, encaps with H(pk) at hand   A = 1 (G2), seed
 struct Exchange {
   uint2 msg[2][3][17], raw[2][3][17];
 };
-enum Role : int { R_KEYPAIR, R_ENC, R_DEC, R_ABSORB };
+enum Role : int { R_KEYPAIR, R_ENC, R_ENC_PKH, R_DEC };
 
 template <int ROLE>
 struct Steps {
-  static constexpr int A = ROLE == R_ENC || ROLE == R_ABSORB ? 115 : 1;
-  static constexpr int K = ROLE == R_ENC ? 2 : ROLE == R_DEC ? 1 : 0;  // hashes after the first
-  static constexpr int op = ROLE == R_KEYPAIR ? OP_KEYPAIR : ROLE == R_ENC ? OP_ENC : OP_DEC;
+  static constexpr int A = ROLE == R_ENC ? 115 : 1;
+  static constexpr int K = ROLE == R_ENC ? 2 : ROLE == R_KEYPAIR ? 0 : 1;  // hashes after the first
+  static constexpr int op = ROLE == R_KEYPAIR ? OP_KEYPAIR : ROLE == R_DEC ? OP_DEC : OP_ENC;
   // step after which squeezed block 0 is there
   static constexpr int FIRST = A + 2 * K - 1;
 };
-static_assert(PK / 136 + 1 == 115 && CT / 136 == 115, "absorbed blocks");
+static_assert(PK / 136 + 1 == 115, "absorbed blocks");
 
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+// Barrier of chain warp w and its helper.  A barrier number in a register makes the kernel
+// reserve all 16 (four blocks per SM); with two chain warps the numbers are constants.
+template <bool TWO>
+__device__ __forceinline__ void pair_sync(int w) {
+  if (!TWO) asm volatile("bar.sync %0, 64;" ::"r"(1 + w) : "memory");
+  else if (w) asm volatile("bar.sync 2, 64;" ::: "memory");
+  else asm volatile("bar.sync 1, 64;" ::: "memory");
+}
 
-template <int ROLE>
+template <int ROLE, bool TWO>
 __device__ __forceinline__ void chain_warp(const FrodoBatch &b, int first, int squeezes, bool keep, Exchange &x,
                                            uint8_t *xbuf, int bar) {
   using T = Steps<ROLE>;
@@ -191,7 +198,7 @@ __device__ __forceinline__ void chain_warp(const FrodoBatch &b, int first, int s
   msp::zero<S>(a);
   const int steps = T::FIRST + 1 + squeezes;
   for (int t = 0; t < steps; t++) {
-    pair_sync(bar);
+    pair_sync<TWO>(bar);
     const int u = t - T::A;
     const bool later = u >= 0 && u < 2 * T::K;
     if (later && !(u & 1)) continue;
@@ -206,7 +213,7 @@ __device__ __forceinline__ void chain_warp(const FrodoBatch &b, int first, int s
     for (int y = 0; y < 4; y++)
       if (s.lane(y) < 17) s.store(reinterpret_cast<uint8_t *>(&x.raw[t & 1][g][s.lane(y)]), a[y]);
   }
-  pair_sync(bar);
+  pair_sync<TWO>(bar);
   if (keep) {
     const int i = first + g;
     const bool live = i < b.n;
@@ -222,10 +229,9 @@ __device__ __forceinline__ uint2 first_message(const Inst &v, int t, int q) {
     const int m = 17 * t + q;
     return m < PK / 8 ? ld_lane(v.pk + 8 * m) : make_uint2(0x1Fu, kEnd);
   }
-  if (ROLE == R_ABSORB) return ld_lane(v.ct + 8 * (17 * t + q));
-  if (ROLE == R_DEC) {  // pkh || mu'
-    if (q < 3) return ld_lane(v.sk + SK_PKH + 8 * q);
-    if (q < 6) return ld_lane(v.mu + 8 * (q - 3));
+  if (ROLE == R_DEC || ROLE == R_ENC_PKH) {  // pkh || mu
+    if (q < 3) return ld_lane((ROLE == R_DEC ? v.sk + SK_PKH : v.pkh) + 8 * q);
+    if (q < 6) return ld_lane((ROLE == R_DEC ? v.mu : v.coins) + 8 * (q - 3));
     return make_uint2(q == 6 ? 0x1Fu : 0u, q == 16 ? kEnd : 0u);
   }
   return make_uint2(0u, 0u);  // keypair: see seed_message
@@ -243,7 +249,7 @@ __device__ __forceinline__ uint2 seed_message(uint32_t dom, int q, F lane) {
   return w;
 }
 
-template <int ROLE>
+template <int ROLE, bool TWO>
 __device__ __forceinline__ void helper_warp(const FrodoBatch &b, int first, int words, Exchange &x, int bar) {
   using T = Steps<ROLE>;
   const int lane = threadIdx.x & 31;
@@ -265,8 +271,7 @@ __device__ __forceinline__ void helper_warp(const FrodoBatch &b, int first, int 
       } else if (t < T::A) {
         w = first_message<ROLE>(v, t, q);
       } else if (ROLE == R_ENC && t == T::A + 1) {  // G2: pkh || mu
-        w = q < 3 ? (v.pkh ? ld_lane(v.pkh + 8 * q) : out(q)) : q < 6 ? ld_lane(v.coins + 8 * (q - 3))
-                                                                  : make_uint2(q == 6 ? 0x1Fu : 0u, q == 16 ? 0x80000000u : 0u);
+        w = q < 3 ? out(q) : q < 6 ? ld_lane(v.coins + 8 * (q - 3)) : make_uint2(q == 6 ? 0x1Fu : 0u, q == 16 ? 0x80000000u : 0u);
       } else {  // 0x96 || seedSE
         w = seed_message(0x96u, q, out);
       }
@@ -275,7 +280,6 @@ __device__ __forceinline__ void helper_warp(const FrodoBatch &b, int first, int 
   };
   // what step t left in raw[t & 1]
   auto consume = [&](int t) {
-    if (ROLE == R_ABSORB) return;
     const int blk = t - T::FIRST;
     if (blk < 0) {
       if (t != T::FIRST - 2 || ROLE == R_KEYPAIR) return;
@@ -300,7 +304,7 @@ __device__ __forceinline__ void helper_warp(const FrodoBatch &b, int first, int 
   prepare(0);
   const int steps = T::FIRST + 1 + max(0, (words + 67) / 68 - 1);
   for (int t = 0; t < steps; t++) {
-    pair_sync(bar);
+    pair_sync<TWO>(bar);
     if (t > 0) consume(t - 1);
     const int u = t + 1;
     if (u < T::A || (u <= T::FIRST && ((u - T::A) & 1))) {
@@ -308,14 +312,48 @@ __device__ __forceinline__ void helper_warp(const FrodoBatch &b, int first, int 
       prepare(u);
     }
   }
-  pair_sync(bar);
+  pair_sync<TWO>(bar);
   consume(steps - 1);
 }
 
+// One block of chains on ten lanes: cw chain warps (three instances each, from block * cw * 3 on) and a
+// helper warp for each, on another SM sub-partition.  HALVE: stop the sampling stream after S'
+// (S^T) and keep its state (tail_kernel goes on).
+template <int ROLE, bool HALVE, bool TWO>
+__device__ __forceinline__ void chain_block(const FrodoBatch &b, int block, int cw, int warp, uint8_t *smem) {
+  constexpr int words = HALVE ? HALF : ROLE == R_KEYPAIR ? 2 * HALF : RW, squeezes = (words + 67) / 68 - 1;
+  const int lane = threadIdx.x & 31;
+  const bool helper = warp >= cw;
+  const int w = helper ? (warp - cw + 2) % cw : warp, first = (block * cw + w) * 3;
+  if (warp >= 2 * cw || first >= b.n) return;
+  Exchange &x = reinterpret_cast<Exchange *>(smem)[w];
+  uint8_t *xbuf = smem + cw * sizeof(Exchange) + w * k10::kSmemPerWarp;
+  if (helper) {
+    if (ROLE == R_DEC && lane < 3 && first + lane < b.n) b.fail[first + lane] = 0;
+    helper_warp<ROLE, TWO>(b, first, words, x, w);
+  } else {
+    chain_warp<ROLE, TWO>(b, first, squeezes, HALVE, x, xbuf, w);
+  }
+}
+constexpr int chain_smem(int cw) { return cw * (int)(sizeof(Exchange) + k10::kSmemPerWarp); }
+static_assert(sizeof(Exchange) % 16 == 0 && k10::kSmemPerWarp % 16 == 0, "16-byte aligned transpose buffers");
+
+// Decaps: the final hash over ct's full blocks, which does not wait for k.  Half as long as the
+// sampling chain, so it runs on lane pairs: 135 integer instructions per state and permutation
+// against the ten lanes' 160, and two shuffles against six shared-memory pipe cycles.
+constexpr int kAbsorbWarps = 4;
+__device__ __forceinline__ void absorb_warp(const FrodoBatch &b, int w) {
+  using S = msp::Multi<2>;
+  const S s(nullptr);
+  const int i = w * S::STATES_PER_WARP + s.state();
+  if (w * S::STATES_PER_WARP >= b.n) return;
+  const bool live = i < b.n;
+  fdev::ct_absorb_multi<S>(inst_of(b, live ? i : b.n - 1, OP_DEC), s, live);
+}
+
 // NS: lanes per state of the sponges (10: ten lanes, 0: one lane, a thread per instance).
-// HALVE: stop the sampling stream after S' (S^T) and keep its state (tail_kernel goes on).
-// Chain blocks run `chain_warps` chain warps each (at most 8), helper warps after them; row
-// blocks [0, early) find an SM at once.
+// Chain blocks run `chain_warps` chain warps each (at most 8); row blocks [0, early) find an SM
+// at once.
 template <int STAGE, int NS, bool HALVE, class G>
 __global__ void __launch_bounds__(32 * kFrontWarps, 1) front_kernel(FrodoBatch b, int chain_warps, int chain_blocks,
                                                                     int absorb_blocks, int early) {
@@ -348,28 +386,28 @@ __global__ void __launch_bounds__(32 * kFrontWarps, 1) front_kernel(FrodoBatch b
       fdev::kp_prologue_inst(v, park, 32 * kFrontWarps);
     }
   } else {
-    // chain warp w's helper is on another SM sub-partition than w
-    const int cw = absorb ? 8 : chain_warps;
-    const bool helper = warp >= cw;
-    const int w = helper ? (warp - cw + 2) % cw : warp, first = (block * cw + w) * 3;
-    if (warp >= 2 * cw || first >= b.n) return;
-    Exchange &x = reinterpret_cast<Exchange *>(smem)[w];
-    uint8_t *xbuf = smem + 8 * sizeof(Exchange) + w * k10::kSmemPerWarp;
-    constexpr int role = STAGE == F_KEYPAIR ? R_KEYPAIR : STAGE == F_ENC ? R_ENC : R_DEC;
-    constexpr int words = HALVE ? HALF : STAGE == F_KEYPAIR ? 2 * HALF : RW, squeezes = (words + 67) / 68 - 1;
     if (absorb) {
-      if constexpr (STAGE == F_DEC) {
-        if (helper) helper_warp<R_ABSORB>(b, first, 0, x, 1 + w);
-        else chain_warp<R_ABSORB>(b, first, 0, true, x, xbuf, 1 + w);
-      }
-    } else if (helper) {
-      if (STAGE == F_DEC && (threadIdx.x & 31) < 3 && first + (int)(threadIdx.x & 31) < b.n)
-        b.fail[first + (threadIdx.x & 31)] = 0;
-      helper_warp<role>(b, first, words, x, 1 + w);
+      if constexpr (STAGE == F_DEC)
+        if (warp < kAbsorbWarps) absorb_warp(b, block * kAbsorbWarps + warp);
     } else {
-      chain_warp<role>(b, first, squeezes, HALVE, x, xbuf, 1 + w);
+      chain_block<STAGE == F_KEYPAIR ? R_KEYPAIR : STAGE == F_ENC ? R_ENC : R_DEC, HALVE, false>(b, block, chain_warps,
+                                                                                                 warp, smem);
     }
   }
+}
+
+// The chains alone, for batches whose A needs no generating (one key) or runs in another form: two
+// chain and two helper warps a block (small blocks spread evenly over the SMs; odd blocks hold the
+// helpers first, so every sub-partition gets both), decaps' absorb blocks after them.
+template <int ROLE>
+__global__ void __launch_bounds__(128, 6) chains_kernel(FrodoBatch b, int chain_blocks) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, block = blockIdx.x;
+  if (block < chain_blocks) {
+    chain_block<ROLE, false, true>(b, block, 2, (warp + 2 * (block & 1)) & 3, smem);
+    return;
+  }
+  if constexpr (ROLE == R_DEC) absorb_warp(b, (block - chain_blocks) * kAbsorbWarps + warp);
 }
 
 // seedA = SHAKE256(z, 16) into pk, one thread per instance: the front kernel's rows need it.
