@@ -137,6 +137,72 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
 }
 
 
+// ---- stage bodies as calls ----
+// Each body is a function of its own: inlined into one kernel, the compiler allocates registers for all of
+// them together (8.6 KB of spill stores), and a change to one stage moved the spills of the others: the
+// Saber product's new form made a mix of 4,096 requests 14 % slower (7.09 -> 8.08 ms) although that
+// stage is faster; with calls the same mix takes 6.84 ms.
+template <int OP>
+static __device__ __noinline__ void call_frodo_prologue(const fdev::Inst &v) {
+  if constexpr (OP == OP_KEYPAIR) fdev::kp_prologue_inst(v);
+  else fdev::prologue_inst<OP>(v);
+}
+template <int OP>
+static __device__ __noinline__ void call_frodo_hash(const fdev::Inst &v) {
+  if constexpr (OP == OP_KEYPAIR) fdev::pk_hash_inst(v);
+  else fdev::ss_inst<OP>(v);
+}
+static __device__ __noinline__ void call_frodo_absorb(const fdev::Inst &v) { fdev::ct_absorb_inst(v); }
+template <int OP>
+static __device__ __noinline__ void call_frodo_prologue_warp(const fdev::Inst &v) {
+  const msp::Multi<1> s(nullptr);
+  if constexpr (OP == OP_KEYPAIR) fdev::kp_prologue_multi(v, s, true);
+  else fdev::prologue_multi<msp::Multi<1>, OP>(v, s, true);
+}
+template <int OP>
+static __device__ __noinline__ void call_frodo_hash_warp(const fdev::Inst &v) {
+  const msp::Multi<1> s(nullptr);
+  if constexpr (OP == OP_KEYPAIR) fdev::pk_hash_multi(v, s, true);
+  else fdev::ss_multi<msp::Multi<1>, OP>(v, s, true);
+}
+static __device__ __noinline__ void call_frodo_absorb_warp(const fdev::Inst &v) {
+  fdev::ct_absorb_multi(v, msp::Multi<1>(nullptr), true);
+}
+template <int L, int OP>
+static __device__ __noinline__ void call_saber_prologue(const sdev::Inst &v, int role) {
+  sdev::prologue_inst<L, OP>(v, role);
+}
+template <int L, int OP>
+static __device__ __noinline__ void call_saber_finish(const sdev::Inst &v) {
+  sdev::finish_inst<L, OP>(v);
+}
+template <int L, int OP>
+static __device__ __noinline__ void call_saber_prologue_warp(const sdev::Inst &v, int role) {
+  sdev::prologue_multi<msp::Multi<1>, L, OP>(v, msp::Multi<1>(nullptr), role, true);
+}
+template <int L, int OP>
+static __device__ __noinline__ void call_saber_finish_warp(const sdev::Inst &v) {
+  const msp::Multi<1> s(nullptr);
+  if constexpr (OP == OP_KEYPAIR) sdev::finish_kp_multi<msp::Multi<1>, L>(v, s, true);
+  else sdev::finish_enc_multi<msp::Multi<1>, L>(v, s, true);
+}
+template <int L, int MODE, int FORM>
+static __device__ __noinline__ void call_saber_product(const sdev::Inst &v, uint8_t *smem, uint32_t tbase, uint32_t *err) {
+  if constexpr (FORM == FORM_TC) sdev::product_tc_cta<L, MODE>(v, smem, tbase, err);
+  else sdev::product_dp4a_cta<L, MODE, FORM == FORM_INT32>(v, smem);
+}
+template <int OP, int FORM, int NST, class G>
+static __device__ __noinline__ void call_frodo_product(const fdev::Inst &v, uint8_t *smem, uint32_t tbase, uint32_t *err) {
+  if constexpr (OP == OP_KEYPAIR) {
+    if constexpr (FORM == FORM_TC) fdev::kp_as_tc_cta<NST == 2 ? fdev::KPT_NST : 1, G>(v, smem, tbase, err);
+    else fdev::kp_as_dp4a_cta<FORM == FORM_INT32, G>(v, smem);
+  } else {
+    if constexpr (FORM == FORM_TC) fdev::sa_tc_cta<OP, NST, G>(v, smem, tbase, err);
+    else fdev::sa_dp4a_cta<OP, FORM == FORM_INT32, G>(v, smem);
+  }
+}
+static __device__ __noinline__ void call_frodo_dec_w(const fdev::Inst &v, uint8_t *smem) { fdev::dec_w_cta(v, smem); }
+
 template <int L>
 __device__ __forceinline__ void saber_thread(const CoinKey &key, int op, int stage, const DevReq &r, int role) {
   sdev::Inst v = saber_view<L>(r);
@@ -148,22 +214,20 @@ __device__ __forceinline__ void saber_thread(const CoinKey &key, int op, int sta
     v.coins = slot;
   }
   if (op == OP_KEYPAIR) {
-    if (stage == 0) sdev::prologue_inst<L, OP_KEYPAIR>(v, role);
-    else sdev::finish_inst<L, OP_KEYPAIR>(v);
+    if (stage == 0) call_saber_prologue<L, OP_KEYPAIR>(v, role);
+    else call_saber_finish<L, OP_KEYPAIR>(v);
   } else if (op == OP_ENC) {
-    if (stage == 0) sdev::prologue_inst<L, OP_ENC>(v, role);
-    else sdev::finish_inst<L, OP_ENC>(v);
+    if (stage == 0) call_saber_prologue<L, OP_ENC>(v, role);
+    else call_saber_finish<L, OP_ENC>(v);
   } else {
-    if (stage == 1) sdev::prologue_inst<L, OP_DEC>(v, role);
-    else sdev::finish_inst<L, OP_DEC>(v);
+    if (stage == 1) call_saber_prologue<L, OP_DEC>(v, role);
+    else call_saber_finish<L, OP_DEC>(v);
   }
 }
 
 // The same stages on a warp per instance (a warp-wide call: every lane runs it).
 template <int L>
 __device__ __forceinline__ void saber_warp(const CoinKey &key, int op, int stage, const DevReq &r, int role) {
-  using S = msp::Multi<1>;
-  const S s(nullptr);
   sdev::Inst v = saber_view<L>(r);
   if (r.gen && stage == 0 && op != OP_DEC) {
     uint8_t *slot = const_cast<uint8_t *>(r.in0) + (role ? 96 : 0);
@@ -172,37 +236,35 @@ __device__ __forceinline__ void saber_warp(const CoinKey &key, int op, int stage
     v.coins = slot;
   }
   if (op == OP_KEYPAIR) {
-    if (stage == 0) sdev::prologue_multi<S, L, OP_KEYPAIR>(v, s, role, true);
-    else sdev::finish_kp_multi<S, L>(v, s, true);
+    if (stage == 0) call_saber_prologue_warp<L, OP_KEYPAIR>(v, role);
+    else call_saber_finish_warp<L, OP_KEYPAIR>(v);
   } else if (op == OP_ENC) {
-    if (stage == 0) sdev::prologue_multi<S, L, OP_ENC>(v, s, role, true);
-    else sdev::finish_enc_multi<S, L>(v, s, true);
+    if (stage == 0) call_saber_prologue_warp<L, OP_ENC>(v, role);
+    else call_saber_finish_warp<L, OP_ENC>(v);
   } else {
-    if (stage == 1) sdev::prologue_multi<S, L, OP_DEC>(v, s, role, true);
-    else if ((threadIdx.x & 31) == 0) sdev::finish_inst<L, OP_DEC>(v);  // one permutation
+    if (stage == 1) call_saber_prologue_warp<L, OP_DEC>(v, role);
+    else if ((threadIdx.x & 31) == 0) call_saber_finish<L, OP_DEC>(v);  // one permutation
   }
 }
 
 __device__ __forceinline__ void warp_stage(const CoinKey &key, int code, const DevReq &r, int role) {
-  using S = msp::Multi<1>;
   const int scheme = scheme_of(code), op = op_of(code), stage = stage_of(code);
   if (scheme <= 1) {
     if (r.gen && stage == 0 && op != OP_DEC) {
       if ((threadIdx.x & 31) == 0) draw_coins(key, r, const_cast<uint8_t *>(r.in0));
       __syncwarp();
     }
-    const S s(nullptr);
     const fdev::Inst v = frodo_view(r);
     if (op == OP_KEYPAIR) {
-      if (stage == 0) fdev::kp_prologue_multi<S>(v, s, true);
-      else fdev::pk_hash_multi<S>(v, s, true);
+      if (stage == 0) call_frodo_prologue_warp<OP_KEYPAIR>(v);
+      else call_frodo_hash_warp<OP_KEYPAIR>(v);
     } else if (op == OP_ENC) {
-      if (stage == 0) fdev::prologue_multi<S, OP_ENC>(v, s, true);
-      else fdev::ss_multi<S, OP_ENC>(v, s, true);
+      if (stage == 0) call_frodo_prologue_warp<OP_ENC>(v);
+      else call_frodo_hash_warp<OP_ENC>(v);
     } else {
-      if (stage == 1 && role == 0) fdev::prologue_multi<S, OP_DEC>(v, s, true);
-      else if (stage == 1) fdev::ct_absorb_multi<S>(v, s, true);
-      else fdev::ss_multi<S, OP_DEC>(v, s, true);
+      if (stage == 1 && role == 0) call_frodo_prologue_warp<OP_DEC>(v);
+      else if (stage == 1) call_frodo_absorb_warp(v);
+      else call_frodo_hash_warp<OP_DEC>(v);
     }
   } else if (scheme == 2) {
     saber_warp<2>(key, op, stage, r, role);
@@ -219,15 +281,15 @@ __device__ __forceinline__ void thread_stage(const CoinKey &key, int code, const
     if (r.gen && stage == 0 && op != OP_DEC) draw_coins(key, r, const_cast<uint8_t *>(r.in0));
     const fdev::Inst v = frodo_view(r);
     if (op == OP_KEYPAIR) {
-      if (stage == 0) fdev::kp_prologue_inst(v);
-      else fdev::pk_hash_inst(v);
+      if (stage == 0) call_frodo_prologue<OP_KEYPAIR>(v);
+      else call_frodo_hash<OP_KEYPAIR>(v);
     } else if (op == OP_ENC) {
-      if (stage == 0) fdev::prologue_inst<OP_ENC>(v);
-      else fdev::ss_inst<OP_ENC>(v);
+      if (stage == 0) call_frodo_prologue<OP_ENC>(v);
+      else call_frodo_hash<OP_ENC>(v);
     } else {
-      if (stage == 1 && role == 0) fdev::prologue_inst<OP_DEC>(v);
-      else if (stage == 1) fdev::ct_absorb_inst(v);
-      else fdev::ss_inst<OP_DEC>(v);
+      if (stage == 1 && role == 0) call_frodo_prologue<OP_DEC>(v);
+      else if (stage == 1) call_frodo_absorb(v);
+      else call_frodo_hash<OP_DEC>(v);
     }
   } else if (scheme == 2) {
     saber_thread<2>(key, op, stage, r, role);
@@ -241,9 +303,9 @@ __device__ __forceinline__ void thread_stage(const CoinKey &key, int code, const
 template <int L, int MODE>
 __device__ __forceinline__ void saber_product(int form, const sdev::Inst &v, uint8_t *smem, uint32_t tbase,
                                               uint32_t *err) {
-  if (form == FORM_TC) sdev::product_tc_cta<L, MODE>(v, smem, tbase, err);
-  else if (form == FORM_INT32) sdev::product_dp4a_cta<L, MODE, true>(v, smem);
-  else sdev::product_dp4a_cta<L, MODE, false>(v, smem);
+  if (form == FORM_TC) call_saber_product<L, MODE, FORM_TC>(v, smem, tbase, err);
+  else if (form == FORM_INT32) call_saber_product<L, MODE, FORM_INT32>(v, smem, tbase, err);
+  else call_saber_product<L, MODE, FORM_DP4A>(v, smem, tbase, err);
 }
 
 template <int L>
@@ -258,26 +320,24 @@ __device__ __forceinline__ void saber_cta(int op, int stage, int tc, const DevRe
 
 constexpr int kTcStages = 2;
 
-// Frodo CTA stages with row generator GT (tcgen05 stage, NST tile stages) / GD (others).
+// Frodo product of one operation with row generator GT (tcgen05 stage, NST tile stages; keypair: every
+// form) / GD (the other forms).
+template <int OP, class GT, class GD, int NST>
+__device__ __forceinline__ void frodo_product(int form, const fdev::Inst &v, uint8_t *smem, uint32_t tbase,
+                                              uint32_t *err) {
+  if (form == FORM_TC) call_frodo_product<OP, FORM_TC, NST, GT>(v, smem, tbase, err);
+  else if (form == FORM_INT32) call_frodo_product<OP, FORM_INT32, NST, GD>(v, smem, tbase, err);
+  else call_frodo_product<OP, FORM_DP4A, NST, GD>(v, smem, tbase, err);
+}
+
 template <class GT, class GD, int NST>
 __device__ __forceinline__ void frodo_cta(int op, int stage, int tc, const DevReq &r, uint8_t *smem, uint32_t tbase,
                                           uint32_t *err) {
   const fdev::Inst v = frodo_view(r);
-  if (op == OP_KEYPAIR) {
-    if (tc == FORM_TC) fdev::kp_as_tc_cta<NST == 2 ? fdev::KPT_NST : 1, GT>(v, smem, tbase, err);
-    else if (tc == FORM_INT32) fdev::kp_as_dp4a_cta<true, GT>(v, smem);
-    else fdev::kp_as_dp4a_cta<false, GT>(v, smem);
-  } else if (op == OP_ENC) {
-    if (tc == FORM_TC) fdev::sa_tc_cta<OP_ENC, NST, GT>(v, smem, tbase, err);
-    else if (tc == FORM_INT32) fdev::sa_dp4a_cta<OP_ENC, true, GD>(v, smem);
-    else fdev::sa_dp4a_cta<OP_ENC, false, GD>(v, smem);
-  } else if (stage == 0) {
-    fdev::dec_w_cta(v, smem);
-  } else {
-    if (tc == FORM_TC) fdev::sa_tc_cta<OP_DEC, NST, GT>(v, smem, tbase, err);
-    else if (tc == FORM_INT32) fdev::sa_dp4a_cta<OP_DEC, true, GD>(v, smem);
-    else fdev::sa_dp4a_cta<OP_DEC, false, GD>(v, smem);
-  }
+  if (op == OP_KEYPAIR) frodo_product<OP_KEYPAIR, GT, GT, NST>(tc, v, smem, tbase, err);
+  else if (op == OP_ENC) frodo_product<OP_ENC, GT, GD, NST>(tc, v, smem, tbase, err);
+  else if (stage == 0) call_frodo_dec_w(v, smem);
+  else frodo_product<OP_DEC, GT, GD, NST>(tc, v, smem, tbase, err);
 }
 
 __device__ __forceinline__ void cta_stage(int code, const DevReq &r, uint8_t *smem, uint32_t tbase, uint32_t *err) {
@@ -297,8 +357,8 @@ __device__ __forceinline__ void cta_stage(int code, const DevReq &r, uint8_t *sm
 }
 
 constexpr int kSmem = std::max({fdev::TcLayout<kTcStages>::total, fdev::DP4A_SMEM, fdev::DEC_W_SMEM,
-                                fdev::KP_AS_SMEM, fdev::KptLayout::total, sdev::PL<4>::TC_TOTAL, sdev::PL<3>::TC_TOTAL,
-                                sdev::PL<2>::TC_TOTAL,
+                                fdev::KP_AS_SMEM, fdev::KptLayout::total, sdev::PL<4>::DP4A_TOTAL, sdev::PL<3>::DP4A_TOTAL,
+                                sdev::PL<2>::DP4A_TOTAL, sdev::TL<4>::TOTAL, sdev::TL<3>::TOTAL, sdev::TL<2>::TOTAL,
                                 // FrodoKEM-976-AES stages: layout + AES table copies
                                 fdev::TcLayout<1>::total + fdev::AesRowsFull::SMEM,
                                 fdev::DP4A_SMEM + fdev::AesRowsHalf::SMEM, fdev::KP_AS_SMEM + fdev::AesRowsFull::SMEM,

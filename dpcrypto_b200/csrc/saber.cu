@@ -11,6 +11,7 @@ namespace {
 using sdev::inst_of;
 using sdev::PL;
 using sdev::Scr;
+using sdev::TL;
 
 // One lane per state: 32 instances per block; warp 0 the hash chain and GenSecret, warp 1
 // GenMatrix.
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(256) product_dp4a_kernel(SaberBatch b) {
 
 template <int L, int MODE>
 __global__ void __launch_bounds__(256) product_tc_kernel(SaberBatch b) {
-  using Y = PL<L>;
+  using Y = TL<L>;
   extern __shared__ __align__(1024) uint8_t sm[];
   uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + Y::TSLOT);
   if (threadIdx.x < 32) {
@@ -125,13 +126,16 @@ __global__ void __launch_bounds__(256) product_tc_kernel(SaberBatch b) {
 // Persistent tensor-core product: each CTA keeps its TMEM columns and mbarrier across the
 // instances it takes (i = blockIdx.x, + gridDim.x, ...) and loads the next instance's
 // packed operands into registers while the current one is processed, so an instance's
-// global-load latency hides behind the previous instance's work.  The launch bound asks
-// for five resident CTAs per SM (48 registers; shared memory also allows five): the phases
-// of an instance are latency-bound, so a fifth CTA's warps hide more of them (l=3 product
-// stages at 4,096 instances: 0.161 ms at four CTAs of 54 registers, 0.148 ms at five).
+// global-load latency hides behind the previous instance's work.  The launch bound asks for
+// kProductCtas<L> resident CTAs per SM (40 registers at six; FireSaber's shared memory allows four)
+// and the grid never has more: a seventh CTA waits for a whole CTA's share of the batch.  Encaps
+// product, us, 4 / 5 / 6 / 7 CTAs per SM, measured before the last changes to its stores: l = 3, 16,384
+// instances 143 / 142 / 134 / 162; l = 4, 8,192 170 / 242 / 209 / 186.
+template <int L>
+constexpr int kProductCtas = L == 4 ? 4 : 6;
 template <int L, int MODE>
-__global__ void __launch_bounds__(256, 5) product_tc_persistent_kernel(SaberBatch b) {
-  using Y = PL<L>;
+__global__ void __launch_bounds__(256, kProductCtas<L>) product_tc_persistent_kernel(SaberBatch b) {
+  using Y = TL<L>;
   extern __shared__ __align__(1024) uint8_t sm[];
   uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + Y::TSLOT);
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Y::BAR);
@@ -154,18 +158,15 @@ __global__ void __launch_bounds__(256, 5) product_tc_persistent_kernel(SaberBatc
   uint32_t phase = 0;
   bool ok = true;
   for (; i < b.n; i += gridDim.x) {
-    pf.store(sm);  // the staging area is free: the previous instance ended with a CTA barrier
+    pf.store(sm);  // the staging area is free: the previous instance's MMAs have read it
     __syncthreads();
     if (i + (int)gridDim.x < b.n) pf.load(inst_of<L>(b, i + gridDim.x, op));
-    const sdev::Inst v = inst_of<L>(b, i, op);
-    sdev::unpack_operands<L, MODE>(v, sm);
-    __syncthreads();
-    ok = sdev::tc_mma_epilogue<L, MODE>(v, sm, tbase, b.err, phase) && ok;
+    ok = sdev::tc_product<L, MODE>(inst_of<L>(b, i, op), sm, tbase, b.err, phase) && ok;
     phase ^= 1u;
   }
-  if (threadIdx.x == 0 && ok) mbar_inval(bar);
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && ok) mbar_inval(bar);
   if (threadIdx.x < 32) {
     tc_fence_after();
     tmem_dealloc(tbase, 32);
@@ -182,7 +183,7 @@ cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st) {
   using Y = PL<L>;
   cudaError_t e;
   if (form == FORM_TC) {
-    constexpr int bytes = Y::TC_TOTAL;
+    constexpr int bytes = TL<L>::TOTAL;
     const int per_sm = tuning().saber_tc_ctas_per_sm;
     if (per_sm > 0) {
       // persistent: per_sm CTAs per SM, several instances each.  The CTAs never wait on one
@@ -199,7 +200,7 @@ cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st) {
         if ((e = cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         sms = m > 0 ? m : 1;
       }
-      const int grid = std::min(b.n, sms * per_sm);
+      const int grid = std::min(b.n, sms * std::min(per_sm, kProductCtas<L>));
       product_tc_persistent_kernel<L, MODE><<<grid, 256, bytes, st>>>(b);
     } else {
       if ((e = prep(product_tc_kernel<L, MODE>, bytes)) != cudaSuccess) return e;

@@ -445,7 +445,7 @@ __device__ __forceinline__ uint32_t pack_byte(const uint16_t *v, int q, int bits
 }
 
 // ---------------------------------------------------------------- product kernel
-// Shared-memory layout common to both forms.
+// Shared-memory layout of the dp4a / INT32 forms.
 template <int L>
 struct PL {
   static constexpr int NO_MAX = L + 1;
@@ -460,26 +460,44 @@ struct PL {
   static constexpr int SEQ = CM + SN * 2;                     // s8  [L][528] secret sequences
   static constexpr int SEQ_STRIDE = 528;
   static constexpr int COMMON = SEQ + L * SEQ_STRIDE;
-  // tcgen05 form
-  static constexpr int HANK = (COMMON + 127) & ~127;          // [L][62][128]
-  static constexpr int HANK_STRIDE = 62 * 128;
-  static constexpr int BOP = HANK + L * HANK_STRIDE;          // [NPAD/8][K/16][8][16]
-  static constexpr int NPAD = 2 * NO_MAX <= 8 ? 8 : 16;
-  static constexpr int BOP_GROUP = L * SN / 16 * 128;         // bytes per 8-row N group
-  static constexpr int BAR = BOP + (NPAD / 8) * BOP_GROUP;
-  static constexpr int TSLOT = BAR + 8;
-  static constexpr int TC_TOTAL = TSLOT + 8;
-  // Packed operands copied in from global memory before unpacking; the Hankel matrices
-  // are built after the unpack, so the staging area reuses their space.  Each piece is
-  // followed by 8 readable bytes (unpack_smem).
-  static constexpr int ST_A = HANK;                                         // GenMatrix bytes
+  // Packed operands copied in from global memory before unpacking.  Each piece is followed by
+  // 8 readable bytes (unpack_smem).
+  static constexpr int STAGE = (COMMON + 127) & ~127;
+  static constexpr int ST_A = STAGE;                                        // GenMatrix bytes
   static constexpr int ST_S = ST_A + SP<L>::ARAW + 8;                       // GenSecret bytes
   static constexpr int ST_P = ST_S + SP<L>::SRAW + 8;                       // packed b (pk)
   static constexpr int ST_END = ST_P + SP<L>::POLYVECCOMP + 8;
-  static constexpr int ST_SK = HANK;                                        // decaps inner: 13-bit s
+  static constexpr int ST_SK = STAGE;                                       // decaps inner: 13-bit s
   static constexpr int ST_CT = ST_SK + SP<L>::POLYVEC + 8;                  // and the ciphertext
   static constexpr int ST_END_INNER = ST_CT + SP<L>::CT + 8;
   static constexpr int DP4A_TOTAL = ST_END > ST_END_INNER ? ST_END : ST_END_INNER;
+};
+
+// Shared-memory layout of the tcgen05 form.
+template <int L>
+struct TL {
+  static constexpr int SEQ = 0;                               // s8 [L][528]: E_j, see tc_product
+  static constexpr int SEQ_STRIDE = 528;
+  static constexpr int RES = L * SEQ_STRIDE;                  // u16 [L+1][256] rounded results
+  static constexpr int CM = RES + (L + 1) * SN * 2;           // 32 message bytes
+  static constexpr int HANK = (CM + 32 + 127) & ~127;         // [L][62][128]
+  static constexpr int HANK_STRIDE = 62 * 128;
+  // B operand, [NPAD/8][K/16] core matrices of 8 rows x 16 bytes, 144 bytes apart: the sixteen chunks
+  // of a polynomial are stored by sixteen threads at once, 128 bytes apart all in the same banks.
+  static constexpr int BOP = HANK + L * HANK_STRIDE;
+  static constexpr int CHUNK = 144;
+  static constexpr int NPAD = 2 * (L + 1) <= 8 ? 8 : 16;
+  static constexpr int BOP_GROUP = L * SN / 16 * CHUNK;       // bytes per 8-row N group
+  static constexpr int BAR = BOP + (NPAD / 8) * BOP_GROUP;
+  static constexpr int TSLOT = BAR + 8;
+  static constexpr int TOTAL = TSLOT + 8;
+  // Packed operands: unpacked before the Hankel matrices are built, so in their place.
+  static constexpr int ST_A = HANK;
+  static constexpr int ST_S = ST_A + SP<L>::ARAW + 8;
+  static constexpr int ST_P = ST_S + SP<L>::SRAW + 8;
+  static constexpr int ST_SK = HANK;
+  static constexpr int ST_CT = ST_SK + SP<L>::POLYVEC + 8;
+  static_assert(ST_P + SP<L>::POLYVECCOMP + 8 <= BOP && ST_CT + SP<L>::CT + 8 <= BOP, "staging fits the Hankel area");
 };
 
 template <int L, int MODE>
@@ -498,10 +516,9 @@ __device__ __forceinline__ void copy8(uint8_t *dst, const uint8_t *src, int byte
 // memory, instead of up to three byte loads from global memory per coefficient.
 // The packed inputs of one instance as 8-byte words: source in global memory and
 // destination in the staging area.
-template <int L, int MODE>
+template <int L, int MODE, class Y>
 struct Staged {
   using P = SP<L>;
-  using Y = PL<L>;
   static_assert(P::ARAW % 8 == 0 && P::SRAW % 8 == 0 && P::POLYVECCOMP % 8 == 0 && P::POLYVEC % 8 == 0 &&
                     P::CT % 8 == 0,
                 "8-byte staging");
@@ -534,9 +551,9 @@ struct Staged {
 };
 
 // Copy one instance's packed inputs into the staging area (CTA-wide, 8-byte accesses).
-template <int L, int MODE>
+template <int L, int MODE, class Y>
 __device__ __forceinline__ void stage_operands(const Inst &v, uint8_t *sm) {
-  using T = Staged<L, MODE>;
+  using T = Staged<L, MODE, Y>;
   for (int w = threadIdx.x; w < T::WORDS; w += blockDim.x) *T::dst(sm, w) = *T::src(v, w);
 }
 
@@ -544,7 +561,7 @@ __device__ __forceinline__ void stage_operands(const Inst &v, uint8_t *sm) {
 // early, store() into the staging area once it is free.
 template <int L, int MODE>
 struct OperandPrefetch {
-  using T = Staged<L, MODE>;
+  using T = Staged<L, MODE, TL<L>>;
   uint2 r[T::PER_THREAD];
   __device__ __forceinline__ void load(const Inst &v) {
 #pragma unroll
@@ -567,17 +584,16 @@ __device__ __forceinline__ void unpack_operands(const Inst &v, uint8_t *sm);
 
 template <int L, int MODE>
 __device__ __forceinline__ void load_operands(const Inst &v, uint8_t *sm) {
-  stage_operands<L, MODE>(v, sm);
+  stage_operands<L, MODE, PL<L>>(v, sm);
   __syncthreads();
   unpack_operands<L, MODE>(v, sm);
 }
 
-// Unpack the staged inputs (after stage_operands or a prefetch's store, and a CTA barrier).
+// Unpack the staged inputs (after stage_operands and a CTA barrier).
 template <int L, int MODE>
 __device__ __forceinline__ void unpack_operands(const Inst &v, uint8_t *sm) {
   using P = SP<L>;
   using Y = PL<L>;
-  static_assert(Y::DP4A_TOTAL <= Y::TC_TOTAL, "staging must fit the tensor form's layout");
   const int tid = threadIdx.x;
   uint32_t *secw = reinterpret_cast<uint32_t *>(sm + Y::SEC);  // 4 int8 coefficients per word
   uint16_t *a16 = reinterpret_cast<uint16_t *>(sm + Y::A16);
@@ -645,11 +661,9 @@ __device__ __forceinline__ void unpack_operands(const Inst &v, uint8_t *sm) {
   }
 }
 
-// Secret sequences, one 32-bit word (4 int8) per thread step, from the secrets in SEC.
-//   TC  : E_j[e] = s_ext[e - 255], e in [0, 528): -s[e + 1] for e < 255, s[e - 255] for
-//         255 <= e < 511, 0 above (the Hankel generating sequence).
-//   dp4a: R_j[t] = s_ext[255 - t]: s[255 - t] for t < 256, -s[511 - t] below 512, 0 above.
-template <int L, bool TC>
+// Secret sequences of the dp4a form, one 32-bit word (4 int8) per thread step, from the secrets
+// in SEC: R_j[t] = s_ext[255 - t]: s[255 - t] for t < 256, -s[511 - t] below 512, 0 above.
+template <int L>
 __device__ __forceinline__ void build_seq(uint8_t *sm) {
   using Y = PL<L>;
   constexpr int NW = Y::SEQ_STRIDE / 4;  // 132
@@ -659,14 +673,8 @@ __device__ __forceinline__ void build_seq(uint8_t *sm) {
     const int j = x / NW, k = x - j * NW;
     const uint32_t *sw = secw + 64 * j;
     uint32_t e = 0;
-    if (TC) {
-      if (k <= 63) e = neg_bytes(__funnelshift_r(sw[k], k < 63 ? sw[k + 1] : 0u, 8));
-      else if (k <= 127) e = __funnelshift_r(sw[k - 64], k < 127 ? sw[k - 63] : 0u, 8);
-      if (k == 63) e |= sw[0] << 24;
-    } else {
-      if (k < 64) e = __byte_perm(sw[63 - k], 0, 0x0123);
-      else if (k < 128) e = neg_bytes(__byte_perm(sw[127 - k], 0, 0x0123));
-    }
+    if (k < 64) e = __byte_perm(sw[63 - k], 0, 0x0123);
+    else if (k < 128) e = neg_bytes(__byte_perm(sw[127 - k], 0, 0x0123));
     seqw[x] = e;
   }
 }
@@ -682,7 +690,7 @@ __device__ __forceinline__ const uint16_t *pub_poly(const uint8_t *sm, int o, in
   return o < L ? a16 + (o * L + j) * Y::PS : b16 + j * Y::PS;
 }
 
-// Phase 3: rounding, packing / comparison.  res holds the products mod 2^16.
+// Rounding, packing / comparison of the dp4a / INT32 forms.  res holds the products mod 2^16.
 template <int L, int MODE>
 __device__ __forceinline__ void epilogue(const Inst &v, uint8_t *sm) {
   using P = SP<L>;
@@ -752,7 +760,7 @@ __device__ __forceinline__ void product_dp4a_cta(const Inst &v, uint8_t *sm) {
   const int tid = threadIdx.x;
   load_operands<L, MODE>(v, sm);
   __syncthreads();
-  build_seq<L, false>(sm);
+  build_seq<L>(sm);
   __syncthreads();
   const int base = 255 - tid, wb = base >> 2, sh = 8 * (base & 3);
   int acc[NO];
@@ -796,109 +804,319 @@ __device__ __forceinline__ void product_dp4a_cta(const Inst &v, uint8_t *sm) {
 }
 
 // ---------------------------------------------------------------- tcgen05 form
-// TMEM columns [tbase, tbase + 32) must be allocated by the caller; the mbarrier in
-// shared memory is initialised here.  Returns false if the bounded wait expired.
-// From unpacked operands to the stored result: secret sequences, Hankel and B operand
-// tiles, the MMAs (completion on the mbarrier at Y::BAR, parity `phase`), the TMEM
-// read-back and the epilogue.  Returns false if the bounded wait expired.
-template <int L, int MODE>
-__device__ __forceinline__ bool tc_mma_epilogue(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err,
-                                                uint32_t phase);
+// Four barrier-separated phases per instance (256 threads; the packed operands are staged):
+//   1  operands: every thread unpacks 16 coefficients, the public ones straight into the bytes of
+//      the B operand, the secret ones into the sequences E_j (their negatives and themselves)
+//   2  the Hankel core matrices from E_j
+//   3  one thread's MMAs; read-back, rounding (coefficient = thread), results to shared memory
+//   4  packing: 16 results (5 words at 10 bits) per thread, to global memory or compared there
+// What bounds it: the tensor pipe's operand reads.  An MMA step of 128 x 32 bytes of A takes about 45
+// cycles whatever N is (the math itself 6 % of the pipe), 36 steps an encaps at l = 3: two thirds of the
+// time at 16,384 instances, the rest exposed phases of a few hundred cycles.  The form before had 48 steps,
+// eight barriers (u16 polynomials, secret sequences, rounding and byte-wise packing as passes of their
+// own) and 6,470 warp instructions an encaps; this one has four barriers and 3,900.  Product stage of
+// encaps at l = 2 / 3 / 4, 16,384 / 16,384 / 8,192 instances: 137 / 184 / 156 -> 93 / 123 / 111 us.
+//
+// E_j[e] = s_ext[e - 256], e in [0, 512): -s[e] below 256, s[e - 256] above.  T'[i][k'] = s_ext[i + k' - 255]
+// = E[i + k' + 1], so core matrix t = mi + 2 ki has rows H[t][r][c] = E[8 t + r + c + 1].
 
-template <int L, int MODE>
-__device__ __forceinline__ bool product_tc_cta(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err) {
-  using Y = PL<L>;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Y::BAR);
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    fence_mbar_init();
+// 16 fields of BITS bits starting OFF bits into w, as bytes in reversed order: lo[q] holds the low
+// bytes of fields 15 - 4q (byte 0) .. 12 - 4q, hi[q] their upper bits.
+template <int BITS, int OFF>
+__device__ __forceinline__ void reversed_bytes(const uint32_t *w, uint4 &lo, uint4 &hi) {
+  constexpr int NW = (OFF + 16 * BITS + 31) / 32;
+  uint32_t r[NW + 1], l[4], h[4];
+#pragma unroll
+  for (int k = 0; k < NW; k++) r[k] = w[k];
+  r[NW] = 0;
+  auto field = [&](int i) {
+    const int bit = OFF + i * BITS;
+    return __funnelshift_r(r[bit >> 5], r[(bit >> 5) + 1], bit & 31);
+  };
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const uint32_t a = field(15 - 4 * q), b = field(14 - 4 * q), c = field(13 - 4 * q), d = field(12 - 4 * q);
+    const uint32_t ab = prmt(a, b, 0x5140), cd = prmt(c, d, 0x5140);  // low bytes, then second bytes
+    l[q] = prmt(ab, cd, 0x5410);
+    h[q] = prmt(ab, cd, 0x7632) & (((1u << (BITS - 8)) - 1u) * 0x01010101u);
   }
-  load_operands<L, MODE>(v, sm);
-  __syncthreads();
-  const bool ok = tc_mma_epilogue<L, MODE>(v, sm, tbase, err, 0);
-  if (threadIdx.x == 0 && ok) mbar_inval(bar);
-  return ok;
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
 }
 
+// 16 secret coefficients (words q = 0..3 of 4 int8 each) of polynomial j, group g, into E_j.
+template <int L>
+__device__ __forceinline__ void store_secret(uint8_t *sm, int j, int g, uint4 s) {
+  using Y = TL<L>;
+  uint8_t *e = sm + Y::SEQ + j * Y::SEQ_STRIDE + 16 * g;
+  *reinterpret_cast<uint4 *>(e) = make_uint4(neg_bytes(s.x), neg_bytes(s.y), neg_bytes(s.z), neg_bytes(s.w));
+  *reinterpret_cast<uint4 *>(e + SN) = s;
+}
+
+// Phase 1.
 template <int L, int MODE>
-__device__ __forceinline__ bool tc_mma_epilogue(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err,
-                                                uint32_t phase) {
-  using Y = PL<L>;
+__device__ __forceinline__ void tc_operands(uint8_t *sm) {
+  using P = SP<L>;
+  using Y = TL<L>;
+  constexpr int NO = n_out<L, MODE>();
+  constexpr bool INNER = MODE == PM_DEC_INNER;
+  constexpr int NA = INNER ? 0 : L * L * 16, NP = MODE == PM_KEYPAIR ? 0 : L * 16, NS = L * 16;
+  // chunk of 16 columns K of row n: K = 256 j + 255 - c for coefficient c
+  auto store_public = [&](int o, int j, int g, uint4 lo, uint4 hi) {
+    uint8_t *d = sm + Y::BOP + (16 * j + 15 - g) * Y::CHUNK;
+    const int nl = o, nh = o + NO;
+    *reinterpret_cast<uint4 *>(d + (nl >> 3) * Y::BOP_GROUP + (nl & 7) * 16) = lo;
+    *reinterpret_cast<uint4 *>(d + (nh >> 3) * Y::BOP_GROUP + (nh & 7) * 16) = hi;
+  };
+  for (int x = threadIdx.x; x < NA + NP + NS; x += 256) {
+    if (x < NA) {  // A: 13 bits; an odd group starts in the middle of a word
+      const int m = x >> 4, g = x & 15, row = m / L, col = m - row * L;
+      const int o = MODE == PM_KEYPAIR ? col : row, j = MODE == PM_KEYPAIR ? row : col;  // keypair: A^T s
+      const uint32_t *w = reinterpret_cast<const uint32_t *>(sm + Y::ST_A) + 104 * m + 13 * (g >> 1);
+      uint4 lo, hi;
+      if (g & 1) reversed_bytes<EQ, 16>(w + 6, lo, hi);
+      else reversed_bytes<EQ, 0>(w, lo, hi);
+      store_public(o, j, g, lo, hi);
+    } else if (x < NA + NP) {  // b (b' in the inner product): 10 bits
+      const int y = x - NA, j = y >> 4, g = y & 15;
+      uint4 lo, hi;
+      reversed_bytes<EP, 0>(reinterpret_cast<const uint32_t *>(sm + (INNER ? Y::ST_CT : Y::ST_P)) + 5 * y, lo, hi);
+      store_public(NO - 1, j, g, lo, hi);
+    } else {
+      const int y = x - NA - NP, j = y >> 4, g = y & 15;
+      uint4 s;
+      if (INNER) {  // low bytes of the 13-bit fields (|s| < 128), in order
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(sm + Y::ST_SK) + 13 * (y >> 1);
+        uint4 hi;
+        if (g & 1) reversed_bytes<EQ, 16>(w + 6, s, hi);
+        else reversed_bytes<EQ, 0>(w, s, hi);
+        s = make_uint4(prmt(s.w, 0, 0x0123), prmt(s.z, 0, 0x0123), prmt(s.y, 0, 0x0123), prmt(s.x, 0, 0x0123));
+      } else {  // CBD_mu
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(sm + Y::ST_S) + (P::MU / 2) * y;
+        uint32_t o[4];
+        if (P::MU == 8) {  // a coefficient per byte: popcounts of its nibbles side by side
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            uint32_t t = w[q];
+            t = t - ((t >> 1) & 0x55555555u);
+            t = (t & 0x33333333u) + ((t >> 2) & 0x33333333u);
+            o[q] = (((t & 0x0F0F0F0Fu) | 0x80808080u) - ((t >> 4) & 0x0F0F0F0Fu)) ^ 0x80808080u;
+          }
+        } else {
+          constexpr uint32_t hm = (1u << (P::MU / 2)) - 1u;
+          unpack_words<P::MU, 16>(w, [&](int i, uint32_t t) {
+            const uint32_t c = (uint32_t)(__popc(t & hm) - __popc((t >> (P::MU / 2)) & hm)) & 0xFFu;
+            if ((i & 3) == 0) o[i >> 2] = c;
+            else o[i >> 2] |= c << (8 * (i & 3));
+          });
+        }
+        s = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      store_secret<L>(sm, j, g, s);
+    }
+  }
+}
+
+// Phase 2.  Thread (j, r, part): row r of core matrices t = part, part + STEP, ... of secret j.
+template <int L>
+__device__ __forceinline__ void tc_hankel(uint8_t *sm) {
+  using Y = TL<L>;
+  const int r = threadIdx.x & 7, sh = 8 * ((r + 1) & 3);
+  int j = 0, t = threadIdx.x >> 3;
+  while (j < L) {
+    const uint32_t *sw =
+        reinterpret_cast<const uint32_t *>(sm + Y::SEQ + j * Y::SEQ_STRIDE) + 2 * t + ((r + 1) >> 2);
+    const uint32_t x0 = sw[0], x1 = sw[1], x2 = sw[2], x3 = sw[3], x4 = sw[4];
+    *reinterpret_cast<uint4 *>(sm + Y::HANK + j * Y::HANK_STRIDE + t * 128 + r * 16) =
+        make_uint4(__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh), __funnelshift_r(x2, x3, sh),
+                   __funnelshift_r(x3, x4, sh));
+    t += 32;
+    if (t >= 62) {
+      t -= 62;
+      j++;
+    }
+  }
+}
+
+// Packs N results of BITS bits (u16 at v, 16-byte aligned) into N * BITS / 32 words.
+template <int BITS, int N>
+__device__ __forceinline__ void pack_words(const uint16_t *v, uint32_t (&out)[N * BITS / 32]) {
+  uint32_t w[N / 2];
+#pragma unroll
+  for (int q = 0; q < N / 8; q++) {
+    const uint4 x = reinterpret_cast<const uint4 *>(v)[q];
+    w[4 * q] = x.x;
+    w[4 * q + 1] = x.y;
+    w[4 * q + 2] = x.z;
+    w[4 * q + 3] = x.w;
+  }
+#pragma unroll
+  for (int k = 0; k < N * BITS / 32; k++) out[k] = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    const uint32_t x = (i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu;
+    const int bit = i * BITS, k = bit >> 5, sh = bit & 31;
+    out[k] |= x << sh;
+    if (sh + BITS > 32) out[k + 1] |= x >> (32 - sh);
+  }
+}
+
+// Phases 1..4 on staged operands (a CTA barrier after the staging, by the caller); the MMAs'
+// completion is on the mbarrier at TL::BAR, parity `phase`.  TMEM columns [tbase, tbase + 32) must
+// be allocated.  Returns false if the bounded wait expired.  The caller may stage the next
+// instance's operands at once (they go where the Hankel matrices were), not other layouts before a CTA
+// barrier.
+template <int L, int MODE>
+__device__ __forceinline__ bool tc_product(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err, uint32_t phase) {
+  using P = SP<L>;
+  using Y = TL<L>;
   constexpr int NO = n_out<L, MODE>();
   constexpr int NPAD = 2 * NO <= 8 ? 8 : 16;
+  constexpr bool INNER = MODE == PM_DEC_INNER;
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Y::BAR);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  build_seq<L, true>(sm);
+  tc_operands<L, MODE>(sm);
+  uint32_t cm = 0;  // decaps inner: this coefficient's et bits of c_m (before the Hankel matrices take the place)
+  if (INNER) cm = unpack_smem(sm + Y::ST_CT + P::POLYVECCOMP, tid, P::ET);
   __syncthreads();
-  // Hankel core matrices: H_j[t][r][c] = E_j[8t + r + c].  Row r = tid % 8 is fixed per
-  // thread; (j, t) advance by 32 core matrices per step, and 8 consecutive threads write one
-  // 128-byte core matrix.
-  {
-    const int r = tid & 7, sh = 8 * (r & 3);
-    int j = 0, t = tid >> 3;
-    while (j < L) {
-      const uint32_t *sw = reinterpret_cast<const uint32_t *>(sm + Y::SEQ + j * Y::SEQ_STRIDE) + 2 * t + (r >> 2);
-      const uint32_t x0 = sw[0], x1 = sw[1], x2 = sw[2], x3 = sw[3], x4 = sw[4];
-      *reinterpret_cast<uint4 *>(sm + Y::HANK + j * Y::HANK_STRIDE + t * 128 + r * 16) =
-          make_uint4(__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh), __funnelshift_r(x2, x3, sh),
-                     __funnelshift_r(x3, x4, sh));
-      t += 32;
-      if (t >= 62) {
-        t -= 62;
-        j++;
-      }
-    }
-  }
-  // B operand: row n = o + NO*limb, K = 256 j + k', value = limb(P_{o,j}[255 - k']).  One
-  // thread per (row n, 16-column chunk kc): coefficients 255-k0 .. 240-k0 are two aligned
-  // 16-byte reads (8 little-endian pairs); a PRMT turns two pairs into 4 output bytes,
-  // reversed.  Threads n = 0..7 of a chunk write its 128 bytes contiguously.
-  for (int x = tid; x < NPAD * L * (SN / 16); x += 256) {
-    const int n = (x & 7) + 8 * (x / (8 * L * (SN / 16))), kc = (x >> 3) % (L * SN / 16);
-    const int j = kc / (SN / 16), k0 = 16 * (kc % (SN / 16));
-    uint4 out = make_uint4(0, 0, 0, 0);
-    if (n < 2 * NO) {
-      const int o = n % NO;
-      const uint32_t sel = n < NO ? 0x4602u : 0x5713u;  // low / high byte of each coefficient
-      const uint4 *pw = reinterpret_cast<const uint4 *>(pub_poly<L, MODE>(sm, o, j) + 240 - k0);
-      const uint4 w0 = pw[0], w1 = pw[1];  // coefficients 240-k0 .. 247-k0 and 248-k0 .. 255-k0
-      out = make_uint4(prmt(w1.w, w1.z, sel), prmt(w1.y, w1.x, sel), prmt(w0.w, w0.z, sel), prmt(w0.y, w0.x, sel));
-    }
-    *reinterpret_cast<uint4 *>(sm + Y::BOP + (n >> 3) * Y::BOP_GROUP + kc * 128 + (n & 7) * 16) = out;
-  }
+  tc_hankel<L>(sm);
   fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (tid == 0) {
     constexpr uint32_t idesc = idesc_i8(128, NPAD, true, false, false, false);
-    // Base descriptors; a step moves only the start-address field (address / 16, low word).
-    const uint64_t a0 = sdesc(smem_u32(sm + Y::HANK), 256, 128), b0 = sdesc(smem_u32(sm + Y::BOP), 128, Y::BOP_GROUP);
+    // Base descriptors; a step moves only the start-address field (address / 16, low word).  The
+    // B operand's eight-row groups are eight chunks (128 columns of K) apart for the double steps.
+    const uint64_t a0 = sdesc(smem_u32(sm + Y::HANK), 256, 128),
+                   b0 = sdesc(smem_u32(sm + Y::BOP), Y::CHUNK, NPAD == 8 ? 8 * Y::CHUNK : Y::BOP_GROUP);
+    auto step = [&](int d, int ks, int j, int chunk, uint32_t id, uint32_t acc) {
+      mma_i8(tbase + d, a0 + (uint64_t)((j * Y::HANK_STRIDE + 4 * ks * 128) >> 4),
+             b0 + (uint64_t)(((16 * j + chunk) * Y::CHUNK) >> 4), id, acc);
+    };
+    if constexpr (NPAD == 8) {
+      // Rows i + 128 of the Hankel block are rows i, 128 columns on: D[i + 128] = sum over K'' of
+      // E[i + K'' + 1] P[K'' - 128].  With K'' in 0 .. 383 one A tile serves both halves of the
+      // coefficients, as 16 columns where both have terms (lower half in columns 8..15): 12
+      // tiles of A per secret instead of 16.  Reading A (4 KB a step) is what the MMAs cost.
+      constexpr uint32_t id16 = idesc_i8(128, 16, true, false, false, false);
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++)
+      for (int j = 0; j < L; j++) {
 #pragma unroll
-      for (int j = 0; j < L; j++)
+        for (int ks = 8; ks < 12; ks++) step(0, ks, j, 2 * ks - 8, idesc, (j | (ks - 8)) ? 1u : 0u);
 #pragma unroll
-        for (int ks = 0; ks < 8; ks++)
-          mma_i8(tbase + mt * NPAD, a0 + (uint64_t)((j * Y::HANK_STRIDE + (16 * mt + 4 * ks) * 128) >> 4),
-                 b0 + (uint64_t)(((16 * j + 2 * ks) * 128) >> 4), idesc, (j | ks) ? 1u : 0u);
+        for (int ks = 0; ks < 4; ks++) step(8, ks, j, 2 * ks, idesc, (j | ks) ? 1u : 0u);
+#pragma unroll
+        for (int ks = 4; ks < 8; ks++) step(0, ks, j, 2 * ks - 8, id16, 1u);
+      }
+    } else {
+      // Rolled: unrolled, the persistent kernel keeps the descriptors of all 64 steps across its loop,
+      // in spilled registers.
+#pragma unroll 1
+      for (int mj = 0; mj < 2 * L; mj++) {
+        const int mt = mj / L, j = mj - mt * L;
+#pragma unroll
+        for (int ks = 0; ks < 8; ks++) step(mt * NPAD, 4 * mt + ks, j, 2 * ks, idesc, (j | ks) ? 1u : 0u);
+      }
+    }
     mma_commit(bar);
+  }
+  // While the MMAs run: the packing jobs' ciphertext words (comparison), sk's 13-bit secret (keypair).
+  constexpr int NW = EP * 16 / 32;                        // 5 words of 16 results
+  constexpr int VG = P::ET == 4 ? 8 : P::ET == 3 ? 32 : 16, VW = P::ET * VG / 32, VJ = SN / VG;  // c_m: per job
+  const bool pjob = tid < L * 16, vjob = MODE != PM_KEYPAIR && !INNER && tid >= L * 16 && tid < L * 16 + VJ;
+  const int vx = tid - L * 16;
+  uint32_t have[NW];
+  if (MODE == PM_DEC_CMP) {
+    const uint32_t *c = reinterpret_cast<const uint32_t *>(v.ct);
+    if (pjob) {
+#pragma unroll
+      for (int k = 0; k < NW; k++) have[k] = c[NW * tid + k];
+    } else if (vjob) {
+#pragma unroll
+      for (int k = 0; k < VW; k++) have[k] = c[P::POLYVECCOMP / 4 + VW * vx + k];
+    }
+  }
+  if (MODE == PM_KEYPAIR && tid >= 128 && tid < 128 + L * 16) {  // 16 coefficients: 26 bytes
+    const int y = tid - 128;
+    const uint32_t *sw = reinterpret_cast<const uint32_t *>(sm + Y::SEQ + (y >> 4) * Y::SEQ_STRIDE + SN + 16 * (y & 15));
+    uint32_t out[7] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t x = (uint32_t)((int32_t)(sw[i >> 2] << (24 - 8 * (i & 3))) >> 24) & 0x1FFFu;
+      const int bit = i * EQ, k = bit >> 5, sh = bit & 31;
+      out[k] |= x << sh;
+      if (sh + EQ > 32) out[k + 1] |= x >> (32 - sh);
+    }
+    uint16_t *d = reinterpret_cast<uint16_t *>(v.sk + 26 * y);
+#pragma unroll
+    for (int k = 0; k < 13; k++) d[k] = (uint16_t)(out[k >> 1] >> (16 * (k & 1)));
   }
   const bool ok = mbar_wait(bar, phase);
   if (!ok && lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
   tc_fence_after();
-  // Warp w reads TMEM lanes 32 (w % 4) .. of M tile w / 4: coefficient = tid.
+  // Warp w reads TMEM lanes 32 (w % 4) .. of coefficient half w / 4: coefficient = tid.
   uint32_t r[16];
-  tmem_ld16(tbase + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * NPAD, r);
+  tmem_ld16(tbase + ((uint32_t)((warp & 3) * 32) << 16) + (NPAD == 8 ? 8 - 8 * (warp >> 2) : NPAD * (warp >> 2)), r);
   tmem_wait_ld();
+  tc_fence_before();
+  if (INNER) {
+    const uint32_t x = r[0] + (r[1] << 8);
+    const uint32_t m = __ballot_sync(0xffffffffu, ((x + P::H2 - (cm << (EP - P::ET))) >> (EP - 1)) & 1u);
+    if (lane == 0) reinterpret_cast<uint32_t *>(v.scr + Scr<L>::MTXT)[warp] = m;
+    if (tid == 0) *v.fail = 0;  // the re-encryption's comparison ORs into it
+    return ok;
+  }
   uint16_t *res = reinterpret_cast<uint16_t *>(sm + Y::RES);
 #pragma unroll
-  for (int o = 0; o < NO; o++) res[o * SN + tid] = (uint16_t)(r[o] + (r[NO + o] << 8));
-  tc_fence_before();
+  for (int o = 0; o < NO; o++) {
+    const uint32_t x = r[o] + (r[NO + o] << 8) + P::H1;
+    if (MODE == PM_KEYPAIR || o < L) {
+      res[o * SN + tid] = (uint16_t)((x >> (EQ - EP)) & 0x3FFu);
+    } else {
+      const uint32_t mb = (sm[Y::CM + (tid >> 3)] >> (tid & 7)) & 1u;
+      res[o * SN + tid] = (uint16_t)(((x - (mb << (EP - 1))) >> (EP - P::ET)) & ((1u << P::ET) - 1u));
+    }
+  }
   __syncthreads();
-  tc_fence_after();
-  epilogue<L, MODE>(v, sm);
+  uint8_t *dst = MODE == PM_KEYPAIR ? v.pk : v.ct;
+  uint32_t diff = 0;
+  if (pjob) {
+    uint32_t w[NW];
+    pack_words<EP, 16>(res + 16 * tid, w);
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+      if (MODE == PM_DEC_CMP) diff |= w[k] ^ have[k];
+      else reinterpret_cast<uint32_t *>(dst)[NW * tid + k] = w[k];
+    }
+  } else if (vjob) {
+    uint32_t w[VW];
+    pack_words<P::ET, VG>(res + L * SN + VG * vx, w);
+#pragma unroll
+    for (int k = 0; k < VW; k++) {
+      if (MODE == PM_DEC_CMP) diff |= w[k] ^ have[k];
+      else reinterpret_cast<uint32_t *>(dst + P::POLYVECCOMP)[VW * vx + k] = w[k];
+    }
+  }
+  if (MODE == PM_DEC_CMP && __any_sync(0xffffffffu, diff != 0) && lane == 0) atomicOr(v.fail, 1u);
+  return ok;
+}
+
+// One instance on a CTA whose TMEM columns [tbase, tbase + 32) are allocated; the mbarrier is
+// initialised here.
+template <int L, int MODE>
+__device__ __forceinline__ bool product_tc_cta(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err) {
+  using Y = TL<L>;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Y::BAR);
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    fence_mbar_init();
+  }
+  stage_operands<L, MODE, Y>(v, sm);
   __syncthreads();
+  const bool ok = tc_product<L, MODE>(v, sm, tbase, err, 0);
+  __syncthreads();
+  if (threadIdx.x == 0 && ok) mbar_inval(bar);
   return ok;
 }
 
