@@ -105,6 +105,20 @@ __global__ void __launch_bounds__(256, 2) mixed_kernel(Plan p) {
       if (s_ready) cta_stage(code, p.req[r], smem, tbase, p.err);  // skipped after an error: the batch drains
       __syncthreads();
       if (tid == 0) mark_done(p, r);
+    } else if (tk.code & kChainTask) {
+      uint32_t r = 0;
+      int ok = 1;
+      if (tid < tk.count) {
+        r = p.idx[tk.first + tid];
+        ok = wait_done(p, r, need) ? 1 : 0;
+        reinterpret_cast<DevReq *>(smem + kChainReqs)[tid] = p.req[r];
+      }
+      if (__syncthreads_and(ok)) chain_task(p.key, code, tk.count, smem);
+      __syncthreads();
+      if (tid < tk.count) {
+        __threadfence();
+        atomicAdd(p.done + r, kind == K_THREAD2 ? 2u : 1u);
+      }
     } else if (tk.code & kWarpTask) {
       const int warp = tid >> 5, lane = tid & 31;
       const int slot = kind == K_THREAD2 ? warp >> 1 : warp, role = kind == K_THREAD2 ? warp & 1 : 0;
@@ -175,8 +189,16 @@ int task_size(int scheme, int kind) {
 // Whether a thread-level stage of a group of `count` requests runs as warp tasks (a warp
 // per instance), and the instances per task either way.
 bool warp_tasks(int kind, size_t count) { return kind != K_CTA && count <= (size_t)tuning().mixed_warp_max; }
-int task_per(int scheme, int kind, size_t count) {
+// FrodoKEM sponges run as chain tasks (unless the knob asks for warp tasks).  ms for a batch of one
+// operation on threads / chain tasks: encaps 2,048 requests 10.9 / 8.6, 4,096 18.2 / 16.7, 8,192 32.7 /
+// 32.7; the four-scheme mix of 512 4.6 / 1.6, of 4,096 7.4 / 4.8.
+bool chain_tasks(int scheme, int op, int stage, size_t count) {
+  return chain_stage(scheme, op, stage) && !warp_tasks(kind_of(scheme, op, stage), count);
+}
+int task_per(int scheme, int op, int stage, size_t count) {
+  const int kind = kind_of(scheme, op, stage);
   if (kind == K_CTA) return 1;
+  if (chain_tasks(scheme, op, stage, count)) return chain_per(op, stage);
   if (warp_tasks(kind, count)) return kind == K_THREAD2 ? 4 : 8;
   return task_size(scheme, kind);
 }
@@ -194,8 +216,7 @@ size_t plan_bytes(const Req *reqs, size_t n, size_t *ntasks_out) {
       const size_t c = counts[s][op];
       if (!c) continue;
       for (int st = 0; st < nstages(s, op); st++) {
-        const int kind = kind_of(s, op, st);
-        const size_t per = (size_t)task_per(s, kind, c);
+        const size_t per = (size_t)task_per(s, op, st, c);
         ntasks += (c + per - 1) / per;
         nidx += c;
       }
@@ -269,8 +290,8 @@ cudaError_t plan_build(const Req *reqs, size_t n, int form, int slots, uint8_t *
     owner.assign(R.size(), -1);
     for (int stg = 0; stg < nstages(scheme, op); stg++) {
       const int kind = kind_of(scheme, op, stg);
-      const int per = task_per(scheme, kind, R.size());
-      const bool warp = warp_tasks(kind, R.size());
+      const int per = task_per(scheme, op, stg, R.size());
+      const bool chain = chain_tasks(scheme, op, stg, R.size()), warp = !chain && warp_tasks(kind, R.size());
       const uint32_t base = (uint32_t)nid;
       std::memcpy(idx + nid, R.data(), R.size() * 4);
       nid += R.size();
@@ -279,9 +300,10 @@ cudaError_t plan_build(const Req *reqs, size_t n, int form, int slots, uint8_t *
         const int id = (int)ht.size();
         const int lo = owner_prev[a], hi = owner_prev[a + cnt - 1];
         // a warp per instance runs a sponge chain in about half the time of one thread
-        const double dur = est_us(scheme, op, stg, cnt) * (warp ? 0.45 : 1.0);
+        // (on chain tasks in a quarter, beside the product CTAs)
+        const double dur = est_us(scheme, op, stg, cnt) * (chain ? 0.25 : warp ? 0.45 : 1.0);
         const int prio = kind == K_CTA ? (dur > 500 ? 2 : 1) : 0;  // latency-bound thread stages first
-        const int code = code_of(scheme, op, stg, form) | (warp ? kWarpTask : 0);
+        const int code = code_of(scheme, op, stg, form) | (chain ? kChainTask : warp ? kWarpTask : 0);
         ht.push_back(HostTask{Task{(uint16_t)code, (uint16_t)cnt, base + (uint32_t)a}, dur,
                               0.0, lo >= 0 ? hi - lo + 1 : 0, INT32_MAX, -1, prio});
         for (int k = 0; k < cnt; k++) owner[a + k] = id;

@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "coins_dev.cuh"
+#include "frodo_chain.cuh"
 #include "frodo_dev.cuh"
 #include "saber_dev.cuh"
 
@@ -36,6 +37,15 @@ enum Kind : int { K_THREAD = 0, K_CTA = 1, K_THREAD2 = 2 };
 // leave the GPU idle (knob mixed_warp_max).
 constexpr int kWarpTask = 1 << 10;
 static_assert(code_of(4, 3, 7, 3) < kWarpTask, "stage codes must stay below the warp-task flag");
+
+// A FrodoKEM prologue or hash stage on ten lanes per state (frodo_chain.cuh): a task is as many
+// instances as one CTA's warps take at once, so a request's 232-348 dependent permutations cost 0.5-0.8 ms
+// instead of the 2-3 ms of one thread beside the product CTAs.
+constexpr int kChainTask = 1 << 11;
+__host__ __device__ constexpr bool chain_stage(int scheme, int op, int stage) {
+  return scheme <= 1 && (op == OP_DEC ? stage == 1 : stage != 1);
+}
+__host__ __device__ constexpr int chain_per(int op, int stage) { return op == OP_DEC ? 6 : stage == 0 ? 12 : 24; }
 
 __host__ __device__ constexpr int nstages(int scheme, int op) { return op == OP_DEC ? 4 : 3; }
 
@@ -203,6 +213,78 @@ static __device__ __noinline__ void call_frodo_product(const fdev::Inst &v, uint
 }
 static __device__ __noinline__ void call_frodo_dec_w(const fdev::Inst &v, uint8_t *smem) { fdev::dec_w_cta(v, smem); }
 
+// Requests of a chain task, copied to shared memory.
+struct ReqInsts {
+  const DevReq *rq;
+  int n;
+  __device__ __forceinline__ fdev::Inst operator()(int i) const { return frodo_view(rq[i]); }
+};
+
+template <int ROLE, int CW>
+__device__ __forceinline__ void frodo_chain(const ReqInsts &src, uint8_t *smem) {
+  using namespace fchain;
+  const int warp = threadIdx.x >> 5;
+  if (warp >= 2 * CW) return;
+  const bool helper = warp >= CW;
+  const int w = helper ? (warp - CW + 2) % CW : warp;
+  if (3 * w >= src.n) return;
+  constexpr int words = ROLE == R_KEYPAIR ? 2 * HALF : frodo::RW;
+  Exchange &x = reinterpret_cast<Exchange *>(smem)[w];
+  uint8_t *xbuf = smem + 4 * sizeof(Exchange) + w * k10::kSmemPerWarp;
+  if (helper) helper_warp<ROLE, false>(src, 3 * w, words, x, w);
+  else chain_warp<ROLE, false>(src, 3 * w, (words + 67) / 68 - 1, false, x, xbuf, w);
+}
+
+// One chain task (the whole CTA, 256 threads).
+template <int OP>
+static __device__ __noinline__ void call_frodo_chain(const ReqInsts &src, uint8_t *smem) {
+  if constexpr (OP == OP_KEYPAIR) {
+    if ((int)threadIdx.x < src.n) fchain::write_seed_a(src(threadIdx.x));
+    __syncthreads();
+    frodo_chain<fchain::R_KEYPAIR, 4>(src, smem);
+  } else if constexpr (OP == OP_ENC) {
+    frodo_chain<fchain::R_ENC, 4>(src, smem);
+  } else {
+    const int warp = threadIdx.x >> 5;
+    frodo_chain<fchain::R_DEC, 2>(src, smem);
+    if (warp >= 4 && 3 * (warp - 4) < src.n) {  // the ciphertext's part of the final hash
+      using S = msp::Multi<10>;
+      const S s(smem + 4 * sizeof(fchain::Exchange) + warp * S::SMEM_PER_WARP);
+      const int i = 3 * (warp - 4) + s.state();
+      fdev::ct_absorb_multi<S>(src(i < src.n ? i : src.n - 1), s, i < src.n);
+    }
+  }
+}
+template <int OP>
+static __device__ __noinline__ void call_frodo_hash_ten(const ReqInsts &src, uint8_t *smem) {
+  using S = msp::Multi<10>;
+  const int warp = threadIdx.x >> 5;
+  if (3 * warp >= src.n) return;
+  const S s(smem + warp * S::SMEM_PER_WARP);
+  const int i = 3 * warp + s.state();
+  const fdev::Inst v = src(i < src.n ? i : src.n - 1);
+  if constexpr (OP == OP_KEYPAIR) fdev::pk_hash_multi<S>(v, s, i < src.n);
+  else fdev::ss_multi<S, OP>(v, s, i < src.n);
+}
+constexpr int kChainReqs = 32 << 10;  // where a chain task's requests lie in shared memory
+
+__device__ __forceinline__ void chain_task(const CoinKey &key, int code, int count, uint8_t *smem) {
+  const int op = op_of(code), stage = stage_of(code);
+  const ReqInsts src{reinterpret_cast<const DevReq *>(smem + kChainReqs), count};
+  if (stage == 0 && (int)threadIdx.x < count && src.rq[threadIdx.x].gen)
+    draw_coins(key, src.rq[threadIdx.x], const_cast<uint8_t *>(src.rq[threadIdx.x].in0));
+  __syncthreads();
+  if (op == OP_KEYPAIR) {
+    if (stage == 0) call_frodo_chain<OP_KEYPAIR>(src, smem);
+    else call_frodo_hash_ten<OP_KEYPAIR>(src, smem);
+  } else if (op == OP_ENC) {
+    if (stage == 0) call_frodo_chain<OP_ENC>(src, smem);
+    else call_frodo_hash_ten<OP_ENC>(src, smem);
+  } else {
+    call_frodo_chain<OP_DEC>(src, smem);
+  }
+}
+
 template <int L>
 __device__ __forceinline__ void saber_thread(const CoinKey &key, int op, int stage, const DevReq &r, int role) {
   sdev::Inst v = saber_view<L>(r);
@@ -363,6 +445,8 @@ constexpr int kSmem = std::max({fdev::TcLayout<kTcStages>::total, fdev::DP4A_SME
                                 fdev::TcLayout<1>::total + fdev::AesRowsFull::SMEM,
                                 fdev::DP4A_SMEM + fdev::AesRowsHalf::SMEM, fdev::KP_AS_SMEM + fdev::AesRowsFull::SMEM,
                                 fdev::KptLayoutT<1>::total + fdev::AesRowsFull::SMEM});
+static_assert(kChainReqs >= 4 * sizeof(fchain::Exchange) + 8 * k10::kSmemPerWarp && kChainReqs + 24 * sizeof(DevReq) <= kSmem,
+              "a chain task's shared memory");
 static_assert(kSmem == fdev::TcLayout<kTcStages>::total, "the AES stages must not raise the kernel's shared memory");
 
 
