@@ -321,6 +321,9 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
       sb.n = (int)m;
       sb.level = scheme;
       sb.err = c->d_err;
+      sb.aux = c->aux[j];
+      sb.fork = c->fork_ev[j];
+      sb.join = c->join_ev[j];
       switch (op) {
         case OP_KEYPAIR:
           sb.coins = d_in0; sb.pk = d_out0; sb.sk = d_out1;
@@ -482,6 +485,9 @@ int dpkem_ctx_create(dpkem_ctx **out, int device, size_t hbm_budget_bytes) {
     const int prio = greatest + (least - greatest) * j / (kPipeChunks - 1);
     cudaStreamCreateWithPriority(&c->ppipe[j], cudaStreamNonBlocking, prio);
     cudaEventCreateWithFlags(&c->stage_ev[j], cudaEventDisableTiming);
+    cudaStreamCreateWithPriority(&c->aux[j], cudaStreamNonBlocking, prio);
+    cudaEventCreateWithFlags(&c->fork_ev[j], cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&c->join_ev[j], cudaEventDisableTiming);
   }
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->last, cudaEventDisableTiming) != cudaSuccess ||
@@ -553,6 +559,12 @@ int dpkem_ctx_destroy(dpkem_ctx *c) {
       cudaStreamSynchronize(c->ppipe[j]);
       cudaStreamDestroy(c->ppipe[j]);
     }
+    if (c->aux[j]) {
+      cudaStreamSynchronize(c->aux[j]);
+      cudaStreamDestroy(c->aux[j]);
+    }
+    if (c->fork_ev[j]) cudaEventDestroy(c->fork_ev[j]);
+    if (c->join_ev[j]) cudaEventDestroy(c->join_ev[j]);
     if (c->stage_ev[j]) {
       cudaEventSynchronize(c->stage_ev[j]);
       cudaEventDestroy(c->stage_ev[j]);

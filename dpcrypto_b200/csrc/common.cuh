@@ -117,6 +117,11 @@ struct SaberBatch {
   uint32_t *fail;        // scratch [n]
   uint32_t *err;         // device error word (DEV_ERR_*)
   StageTimer *timer;     // optional
+  // Decaps: a second stream and two events of the context's, for the sponge that does not
+  // wait for the inner product; null: one stage after the other.
+  cudaStream_t aux;
+  cudaEvent_t fork, join;
+  int sliced;            // set by the launcher: the XOF bytes are in bit-interleaved halves
 };
 
 struct CoinsBatch {

@@ -18,6 +18,8 @@ struct dpkem_ctx {
   cudaStream_t pipe[16] = {};   // host-mode copy/compute pipeline, one stream per chunk
   cudaStream_t ppipe[16] = {};  // the same with descending priorities (chunk 0 highest)
   cudaEvent_t pev[16] = {};
+  cudaStream_t aux[16] = {};    // a second stream per pipeline slot and its fork / join events
+  cudaEvent_t fork_ev[16] = {}, join_ev[16] = {};
   uint8_t *arena = nullptr;
   size_t arena_bytes = 0;
   uint32_t *d_err = nullptr;

@@ -224,15 +224,17 @@ __device__ __forceinline__ void absorb_finish(typename S::W (&a)[S::NS], const S
   s.perm(a);
 }
 
-// Squeeze `len` bytes (a multiple of 8) of a finished state to dst.
-template <class S, int RATE>
+// Squeeze `len` bytes (a multiple of 8) of a finished state to dst.  RAW: each 64-bit word in the
+// layout's form, which a bit-interleaved layout stores as its halves {even, odd} (k10::lane_of
+// restores it), sparing the chain the conversions.
+template <class S, int RATE, bool RAW = false>
 __device__ __forceinline__ void squeeze(typename S::W (&a)[S::NS], const S &s, uint8_t *dst, int len, bool live) {
   constexpr int W = RATE / 8;
   for (int off = 0;; off += RATE) {
     typename S::W w[S::NS];
 #pragma unroll
     for (int y = 0; y < S::NS; y++)
-      if (S::least(y) < W) w[y] = s.out(a[y]);
+      if (S::least(y) < W) w[y] = RAW ? a[y] : s.out(a[y]);
 #pragma unroll
     for (int y = 0; y < S::NS; y++)
       if (S::least(y) < W) pin(w[y]);

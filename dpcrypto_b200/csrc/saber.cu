@@ -13,44 +13,62 @@ using sdev::PL;
 using sdev::Scr;
 using sdev::TL;
 
-// One lane per state: 32 instances per block; warp 0 the hash chain and GenSecret, warp 1
-// GenMatrix.
+// Prologue kernels: role 0 is the hash chain and GenSecret, role 1 GenMatrix.  A launch runs both, a
+// warp each (roles = 2, first = 0), or the one `first` names.
+//
+// One lane per state: 32 instances per block.
 template <int L, int OP>
-__global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b) {
+__global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b, int first) {
   const int i = blockIdx.x * 32 + (threadIdx.x & 31);
-  if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), threadIdx.x >> 5);
+  if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), first + (threadIdx.x >> 5));
 }
 
 // Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 10: ten lanes, three
-// instances per warp; NS = 2: a pair, sixteen).  Two warps per block: warp 0 the hash chain and GenSecret, warp 1
-// GenMatrix, for the same instances.
+// instances per warp; NS = 2: a pair, sixteen).  The bit-interleaved ones leave the XOF bytes in
+// their form (b.sliced): converted there, a pair's 21 words a permutation made the l = 3 prologue of
+// 4,096 85 us against 77, and ten lanes' FireSaber prologue of 1,501 120 against 107; in the product's
+// staging they are two words a thread (2 us).
 template <int L, int OP, int NS>
-__global__ void __launch_bounds__(64) prologue_multi_kernel(SaberBatch b) {
+__global__ void __launch_bounds__(64) prologue_multi_kernel(SaberBatch b, int first) {
   using S = msp::Multi<NS>;
   __shared__ __align__(16) uint8_t xbuf[2 * (S::SMEM_PER_WARP > 0 ? S::SMEM_PER_WARP : 16)];
   const int w = threadIdx.x >> 5;
   const S s(xbuf + w * S::SMEM_PER_WARP);
   const int g = s.state(), i = blockIdx.x * S::STATES_PER_WARP + g;
   const bool live = g < S::STATES_PER_WARP && i < b.n;
-  sdev::prologue_multi<S, L, OP>(inst_of<L>(b, live ? i : b.n - 1, OP), s, w, live);
-}
-
-template <int L, int OP, int NS>
-void launch_prologue_multi(const SaberBatch &b, cudaStream_t st) {
-  constexpr int spw = msp::Multi<NS>::STATES_PER_WARP;
-  prologue_multi_kernel<L, OP, NS><<<(b.n + spw - 1) / spw, 64, 0, st>>>(b);
+  sdev::prologue_multi<S, L, OP, NS != 1>(inst_of<L>(b, live ? i : b.n - 1, OP), s, first + w, live);
 }
 
 // Lanes per state of the prologue's sponges for a batch of n: a warp per state up to
 // saber_warp_max, ten lanes up to saber_five_max (the knob's name is from a layout of five), a
 // pair up to saber_pair_max, else one.
+int prologue_lanes(int n) {
+  const Tuning &t = tuning();
+  return n <= t.saber_warp_max ? 25 : n <= t.saber_five_max ? 10 : n <= t.saber_pair_max ? 2 : 1;
+}
+
+// Whether decaps runs GenMatrix on a second stream beside the inner product and the chain that needs
+// its m'.  It pays while every chain warp finds an SM with little else on it (up to 100
+// blocks), and again when the chains fill the chip several times over; between, the chains slow down
+// next to the product's CTAs by more than the inner product takes, and LightSaber's chain is too short.
+// us, one stream / two, l = 3: n = 1 76 / 70, 300 83 / 78, 444 84 / 93, 1,500 113 / 116, 8,192 260 / 311,
+// 12,000 413 / 388, 16,384 474 / 448; l = 4: 128 115 / 109, 12,000 669 / 539; l = 2: 128 49 / 51.
+template <int L>
+bool matrix_beside_inner(int n) {
+  const int lanes = prologue_lanes(n);
+  return L > 2 && ((lanes == 25 && n <= 100) || (lanes == 10 && n <= 300) || (lanes == 1 && n >= 12000));
+}
+
 template <int L, int OP>
-void launch_prologue(const SaberBatch &b, cudaStream_t st) {
-  const int pb = (b.n + 31) / 32;
-  if (b.n <= tuning().saber_warp_max) launch_prologue_multi<L, OP, 1>(b, st);
-  else if (b.n <= tuning().saber_five_max) launch_prologue_multi<L, OP, 10>(b, st);
-  else if (b.n <= tuning().saber_pair_max) launch_prologue_multi<L, OP, 2>(b, st);
-  else prologue_kernel<L, OP><<<pb, 64, 0, st>>>(b);
+void launch_prologue(const SaberBatch &b, cudaStream_t st, int first = 0, int roles = 2) {
+  auto blocks = [&](int per) { return (b.n + per - 1) / per; };
+  const int threads = 32 * roles;
+  switch (prologue_lanes(b.n)) {
+    case 25: prologue_multi_kernel<L, OP, 1><<<b.n, threads, 0, st>>>(b, first); break;
+    case 10: prologue_multi_kernel<L, OP, 10><<<blocks(3), threads, 0, st>>>(b, first); break;
+    case 2: prologue_multi_kernel<L, OP, 2><<<blocks(16), threads, 0, st>>>(b, first); break;
+    default: prologue_kernel<L, OP><<<blocks(32), threads, 0, st>>>(b, first);
+  }
 }
 
 // Encaps / keypair finish on several lanes per state, one warp per block.
@@ -98,7 +116,7 @@ __host__ __device__ constexpr int op_of(int mode) {
 template <int L, int MODE, bool I32>
 __global__ void __launch_bounds__(256) product_dp4a_kernel(SaberBatch b) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  sdev::product_dp4a_cta<L, MODE, I32>(inst_of<L>(b, blockIdx.x, op_of(MODE)), sm);
+  sdev::product_dp4a_cta<L, MODE, I32>(inst_of<L>(b, blockIdx.x, op_of(MODE)), sm, b.sliced != 0);
 }
 
 template <int L, int MODE>
@@ -114,7 +132,7 @@ __global__ void __launch_bounds__(256) product_tc_kernel(SaberBatch b) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *tslot;
-  sdev::product_tc_cta<L, MODE>(inst_of<L>(b, blockIdx.x, op_of(MODE)), sm, tbase, b.err);
+  sdev::product_tc_cta<L, MODE>(inst_of<L>(b, blockIdx.x, op_of(MODE)), sm, tbase, b.err, b.sliced != 0);
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -158,7 +176,7 @@ __global__ void __launch_bounds__(256, kProductCtas<L>) product_tc_persistent_ke
   uint32_t phase = 0;
   bool ok = true;
   for (; i < b.n; i += gridDim.x) {
-    pf.store(sm);  // the staging area is free: the previous instance's MMAs have read it
+    pf.store(sm, b.sliced != 0);  // the staging area is free: the previous instance's MMAs have read it
     __syncthreads();
     if (i + (int)gridDim.x < b.n) pf.load(inst_of<L>(b, i + gridDim.x, op));
     ok = sdev::tc_product<L, MODE>(inst_of<L>(b, i, op), sm, tbase, b.err, phase) && ok;
@@ -223,7 +241,10 @@ inline void mark(const SaberBatch &b, cudaStream_t st) {
 }
 
 template <int L>
-cudaError_t run(const SaberBatch &b, int op, int form, cudaStream_t st) {
+cudaError_t run(const SaberBatch &batch, int op, int form, cudaStream_t st) {
+  SaberBatch b = batch;
+  const int lanes = prologue_lanes(b.n);
+  b.sliced = lanes == 10 || lanes == 2;
   const int tb = tuning().thread_block;
   const int fb = (b.n + tb - 1) / tb;
   cudaError_t e;
@@ -244,9 +265,21 @@ cudaError_t run(const SaberBatch &b, int op, int form, cudaStream_t st) {
       if (!launch_finish_multi<L, OP_ENC>(b, st)) finish_kernel<L, OP_ENC><<<fb, tb, 0, st>>>(b);
       break;
     default:
-      if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st)) != cudaSuccess) return e;
-      mark(b, st);
-      launch_prologue<L, OP_DEC>(b, st);
+      if (b.aux && !b.timer && matrix_beside_inner<L>(b.n)) {
+        // GenMatrix needs the seed alone, the other sponges m': it runs beside the inner product and the
+        // hash chain that follows it.
+        if ((e = cudaEventRecord(b.fork, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(b.aux, b.fork, 0)) != cudaSuccess) return e;
+        launch_prologue<L, OP_DEC>(b, b.aux, 1, 1);
+        if ((e = cudaEventRecord(b.join, b.aux)) != cudaSuccess) return e;
+        if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st)) != cudaSuccess) return e;
+        launch_prologue<L, OP_DEC>(b, st, 0, 1);
+        if ((e = cudaStreamWaitEvent(st, b.join, 0)) != cudaSuccess) return e;
+      } else {
+        if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st)) != cudaSuccess) return e;
+        mark(b, st);
+        launch_prologue<L, OP_DEC>(b, st);
+      }
       mark(b, st);
       if ((e = launch_product<L, sdev::PM_DEC_CMP>(b, form, st)) != cudaSuccess) return e;
       mark(b, st);

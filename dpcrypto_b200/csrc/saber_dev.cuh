@@ -223,7 +223,8 @@ __device__ __forceinline__ void prologue_inst(const Inst &v, int role) {
 // lanes (msponge.cuh: S = msp::Multi<1>, a warp per state, msp::Multi<10>, ten lanes, or
 // msp::Multi<2>, a pair): the bytes written are those of prologue_inst / finish_inst.  live = false keeps a
 // state without an instance in step (reads stay in bounds, writes are skipped).
-template <class S, int L, int OP>
+// RAW: the XOF bytes stay in the layout's form (msp::squeeze), the product's staging restores them.
+template <class S, int L, int OP, bool RAW = false>
 __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int role, bool live) {
   using P = SP<L>;
   using Q = Scr<L>;
@@ -241,7 +242,7 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int ro
       msp::absorb_aligned<S, 168>(a, s, 0, src, 32, live);
     }
     msp::absorb_finish<S, 168>(a, s, 32, 0x1Fu);
-    msp::squeeze<S, 168>(a, s, scr + Q::ARAW, P::ARAW, live);
+    msp::squeeze<S, 168, RAW>(a, s, scr + Q::ARAW, P::ARAW, live);
     return;
   }
   if (OP == OP_KEYPAIR) {
@@ -273,7 +274,7 @@ __device__ __forceinline__ void prologue_multi(const Inst &v, const S &s, int ro
     msp::xor_lane<S, 3>(a, s, s.template get<7>(kr));
   }
   msp::absorb_finish<S, 168>(a, s, 32, 0x1Fu);
-  msp::squeeze<S, 168>(a, s, scr + Q::SRAW, P::SRAW, live);
+  msp::squeeze<S, 168, RAW>(a, s, scr + Q::SRAW, P::SRAW, live);
   if (OP == OP_DEC) {  // H(c) of the input ciphertext (see prologue_inst)
     msp::zero<S>(a);
     const int pos = msp::absorb_aligned<S, 136>(a, s, 0, v.ct, P::CT, live);
@@ -531,6 +532,10 @@ struct Staged {
   static constexpr int W3 = (INNER || MODE == PM_KEYPAIR) ? 0 : 4;
   static constexpr int WORDS = W0 + W1 + W2 + W3;
   static constexpr int PER_THREAD = (WORDS + 255) / 256;  // with 256 threads
+  // Word w of the XOF bytes, which the prologue may have left as bit-interleaved halves.
+  __device__ __forceinline__ static uint2 natural(int w, uint2 x, bool sliced) {
+    return !INNER && sliced && w < W0 + W1 ? k10::lane_of(x) : x;
+  }
   __device__ __forceinline__ static const uint2 *src(const Inst &v, int w) {
     if (INNER)
       return w < W0 ? reinterpret_cast<const uint2 *>(v.sk) + w : reinterpret_cast<const uint2 *>(v.ct) + (w - W0);
@@ -552,9 +557,9 @@ struct Staged {
 
 // Copy one instance's packed inputs into the staging area (CTA-wide, 8-byte accesses).
 template <int L, int MODE, class Y>
-__device__ __forceinline__ void stage_operands(const Inst &v, uint8_t *sm) {
+__device__ __forceinline__ void stage_operands(const Inst &v, uint8_t *sm, bool sliced) {
   using T = Staged<L, MODE, Y>;
-  for (int w = threadIdx.x; w < T::WORDS; w += blockDim.x) *T::dst(sm, w) = *T::src(v, w);
+  for (int w = threadIdx.x; w < T::WORDS; w += blockDim.x) *T::dst(sm, w) = T::natural(w, *T::src(v, w), sliced);
 }
 
 // The same copy split in two for a persistent loop (256 threads): load() into registers
@@ -570,11 +575,11 @@ struct OperandPrefetch {
       if (w < T::WORDS) r[k] = *T::src(v, w);
     }
   }
-  __device__ __forceinline__ void store(uint8_t *sm) const {
+  __device__ __forceinline__ void store(uint8_t *sm, bool sliced) const {
 #pragma unroll
     for (int k = 0; k < T::PER_THREAD; k++) {
       const int w = threadIdx.x + 256 * k;
-      if (w < T::WORDS) *T::dst(sm, w) = r[k];
+      if (w < T::WORDS) *T::dst(sm, w) = T::natural(w, r[k], sliced);
     }
   }
 };
@@ -583,8 +588,8 @@ template <int L, int MODE>
 __device__ __forceinline__ void unpack_operands(const Inst &v, uint8_t *sm);
 
 template <int L, int MODE>
-__device__ __forceinline__ void load_operands(const Inst &v, uint8_t *sm) {
-  stage_operands<L, MODE, PL<L>>(v, sm);
+__device__ __forceinline__ void load_operands(const Inst &v, uint8_t *sm, bool sliced) {
+  stage_operands<L, MODE, PL<L>>(v, sm, sliced);
   __syncthreads();
   unpack_operands<L, MODE>(v, sm);
 }
@@ -754,11 +759,11 @@ __device__ __forceinline__ void epilogue(const Inst &v, uint8_t *sm) {
 // I32 = true is the INT32 schoolbook form (SABER-GPU/src/poly.cu:209-358, the reference's
 // mode 1): the same window, one 32-bit multiply-add per coefficient pair instead of dp2a.
 template <int L, int MODE, bool I32 = false>
-__device__ __forceinline__ void product_dp4a_cta(const Inst &v, uint8_t *sm) {
+__device__ __forceinline__ void product_dp4a_cta(const Inst &v, uint8_t *sm, bool sliced = false) {
   using Y = PL<L>;
   constexpr int NO = n_out<L, MODE>();
   const int tid = threadIdx.x;
-  load_operands<L, MODE>(v, sm);
+  load_operands<L, MODE>(v, sm, sliced);
   __syncthreads();
   build_seq<L>(sm);
   __syncthreads();
@@ -1105,14 +1110,15 @@ __device__ __forceinline__ bool tc_product(const Inst &v, uint8_t *sm, uint32_t 
 // One instance on a CTA whose TMEM columns [tbase, tbase + 32) are allocated; the mbarrier is
 // initialised here.
 template <int L, int MODE>
-__device__ __forceinline__ bool product_tc_cta(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err) {
+__device__ __forceinline__ bool product_tc_cta(const Inst &v, uint8_t *sm, uint32_t tbase, uint32_t *err,
+                                               bool sliced = false) {
   using Y = TL<L>;
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Y::BAR);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
   }
-  stage_operands<L, MODE, Y>(v, sm);
+  stage_operands<L, MODE, Y>(v, sm, sliced);
   __syncthreads();
   const bool ok = tc_product<L, MODE>(v, sm, tbase, err, 0);
   __syncthreads();
