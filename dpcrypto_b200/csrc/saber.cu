@@ -3,6 +3,7 @@
 // the persistent mixed-batch kernel); these wrappers only map blockIdx/threadIdx to instances.
 #include <algorithm>
 
+#include "saber_chain.cuh"
 #include "saber_dev.cuh"
 
 namespace dpkem {
@@ -13,12 +14,39 @@ using sdev::PL;
 using sdev::Scr;
 using sdev::TL;
 
+// The stages of a call follow one another at once: each kernel lets the next one's blocks start when
+// all of its own have, and waits for its predecessor's results itself (programmatic dependent launch), so
+// launch latency and a kernel's set-up pass while the predecessor drains.  The first kernel of a call is
+// launched plainly and waits for the whole stream.  Only up to kFollowMax instances: a waiting kernel
+// that fills the SMs keeps the next call's sponges, or a persistent product's CTAs, off them.  us, plain /
+// following, encaps at l = 3: n = 1 80 / 74, 444 86 / 82, 600 89 / 88, 1,501 112 / 140, 4,096 149 / 202.
+constexpr int kFollowMax = 512;
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_next(bool follows, void (*kernel)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = follows ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Prologue kernels: role 0 is the hash chain and GenSecret, role 1 GenMatrix.  A launch runs both, a
 // warp each (roles = 2, first = 0), or the one `first` names.
 //
 // One lane per state: 32 instances per block.
 template <int L, int OP>
 __global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b, int first) {
+  next_may_start();
+  wait_predecessor();
   const int i = blockIdx.x * 32 + (threadIdx.x & 31);
   if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), first + (threadIdx.x >> 5));
 }
@@ -30,13 +58,64 @@ __global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b, int first) {
 // staging they are two words a thread (2 us).
 template <int L, int OP, int NS>
 __global__ void __launch_bounds__(64) prologue_multi_kernel(SaberBatch b, int first) {
+  next_may_start();
+  wait_predecessor();
   using S = msp::Multi<NS>;
   __shared__ __align__(16) uint8_t xbuf[2 * (S::SMEM_PER_WARP > 0 ? S::SMEM_PER_WARP : 16)];
   const int w = threadIdx.x >> 5;
   const S s(xbuf + w * S::SMEM_PER_WARP);
   const int g = s.state(), i = blockIdx.x * S::STATES_PER_WARP + g;
   const bool live = g < S::STATES_PER_WARP && i < b.n;
-  sdev::prologue_multi<S, L, OP, NS != 1>(inst_of<L>(b, live ? i : b.n - 1, OP), s, first + w, live);
+  sdev::prologue_multi<S, L, OP, NS == 2>(inst_of<L>(b, live ? i : b.n - 1, OP), s, first + w, live);
+}
+
+// Ten lanes per state on chain and helper warps (saber_chain.cuh), three instances per block: the
+// chains of the roles, then their helpers; odd blocks the other way round, so that every SM
+// sub-partition gets both.
+template <int L, int OP>
+__global__ void __launch_bounds__(128) prologue_chain_kernel(SaberBatch b, int first_role, int roles) {
+  next_may_start();
+  wait_predecessor();
+  using namespace schain;
+  __shared__ Exchange x[2];
+  __shared__ __align__(16) uint8_t xbuf[2][k10::kSmemPerWarp];
+  const int warps = 2 * roles, warp = ((threadIdx.x >> 5) + roles * (blockIdx.x & 1)) & (warps - 1);
+  const int w = warp & (roles - 1), role = first_role + w, first = 3 * blockIdx.x;
+  if (warp < roles) {
+    constexpr Program m = Matrix<L, OP>::prog, s = Secret<L, OP>::prog;
+    const Program p = {role ? m.steps : s.steps, role ? m.msg : s.msg, role ? m.reset : s.reset, role ? m.idle : s.idle};
+    chain_warp(p, x[w], xbuf[w], w);
+  } else {
+    auto inst = [&](int i) { return inst_of<L>(b, i, OP); };
+    if (role) helper_warp<Matrix<L, OP>>(inst, b.n, first, x[w], w);
+    else helper_warp<Secret<L, OP>>(inst, b.n, first, x[w], w);
+  }
+}
+
+// Encaps / keypair finish likewise, 64 threads.
+template <int L, int OP>
+__global__ void __launch_bounds__(64) finish_chain_kernel(SaberBatch b) {
+  next_may_start();
+  wait_predecessor();
+  using namespace schain;
+  __shared__ Exchange x;
+  __shared__ __align__(16) uint8_t xbuf[k10::kSmemPerWarp];
+  const int warp = ((threadIdx.x >> 5) + blockIdx.x) & 1, lane = threadIdx.x & 31, first = 3 * blockIdx.x;
+  if (warp == 0) {
+    constexpr Program p = Finish<L, OP>::prog;
+    chain_warp(p, x, xbuf, 0);
+    return;
+  }
+  auto inst = [&](int i) { return inst_of<L>(b, i, OP); };
+  if (OP == OP_KEYPAIR) {  // sk = s || pk || H(pk) || z: pk and z
+    using P = sdev::SP<L>;
+    for (int i = first; i < first + 3 && i < b.n; i++) {
+      const sdev::Inst v = inst(i);
+      for (int q = lane; q < P::PK / 8; q += 32) put(v.sk + P::POLYVEC + 8 * q, ld_lane(v.pk + 8 * q));
+      if (lane < 4) put(v.sk + P::SK - 32 + 8 * lane, ld_lane(v.coins + 64 + 8 * lane));
+    }
+  }
+  helper_warp<Finish<L, OP>>(inst, b.n, first, x, 0);
 }
 
 // Lanes per state of the prologue's sponges for a batch of n: a warp per state up to
@@ -60,20 +139,22 @@ bool matrix_beside_inner(int n) {
 }
 
 template <int L, int OP>
-void launch_prologue(const SaberBatch &b, cudaStream_t st, int first = 0, int roles = 2) {
+cudaError_t launch_prologue(const SaberBatch &b, cudaStream_t st, bool follows, int first = 0, int roles = 2) {
   auto blocks = [&](int per) { return (b.n + per - 1) / per; };
   const int threads = 32 * roles;
   switch (prologue_lanes(b.n)) {
-    case 25: prologue_multi_kernel<L, OP, 1><<<b.n, threads, 0, st>>>(b, first); break;
-    case 10: prologue_multi_kernel<L, OP, 10><<<blocks(3), threads, 0, st>>>(b, first); break;
-    case 2: prologue_multi_kernel<L, OP, 2><<<blocks(16), threads, 0, st>>>(b, first); break;
-    default: prologue_kernel<L, OP><<<blocks(32), threads, 0, st>>>(b, first);
+    case 25: return launch_next(follows, prologue_multi_kernel<L, OP, 1>, b.n, threads, 0, st, b, first);
+    case 10: return launch_next(follows, prologue_chain_kernel<L, OP>, blocks(3), 2 * threads, 0, st, b, first, roles);
+    case 2: return launch_next(follows, prologue_multi_kernel<L, OP, 2>, blocks(16), threads, 0, st, b, first);
+    default: return launch_next(follows, prologue_kernel<L, OP>, blocks(32), threads, 0, st, b, first);
   }
 }
 
 // Encaps / keypair finish on several lanes per state, one warp per block.
 template <int L, int OP, int NS>
 __global__ void __launch_bounds__(32) finish_multi_kernel(SaberBatch b) {
+  next_may_start();
+  wait_predecessor();
   using S = msp::Multi<NS>;
   __shared__ __align__(16) uint8_t xbuf[S::SMEM_PER_WARP > 0 ? S::SMEM_PER_WARP : 16];
   const S s(xbuf);
@@ -84,29 +165,27 @@ __global__ void __launch_bounds__(32) finish_multi_kernel(SaberBatch b) {
   else sdev::finish_kp_multi<S, L>(v, s, live);
 }
 
-// The finish on a warp, ten lanes or a pair per state when n is within the thresholds; false
-// otherwise.
-template <int L, int OP>
-bool launch_finish_multi(const SaberBatch &b, cudaStream_t st) {
-  if (b.n <= tuning().saber_finish_warp_max) {
-    finish_multi_kernel<L, OP, 1><<<b.n, 32, 0, st>>>(b);
-    return true;
-  }
-  if (b.n <= tuning().saber_finish_five_max) {
-    finish_multi_kernel<L, OP, 10><<<(b.n + 2) / 3, 32, 0, st>>>(b);
-    return true;
-  }
-  if (b.n / 2 <= tuning().saber_pair_max) {  // one sponge per instance, the prologue has two
-    finish_multi_kernel<L, OP, 2><<<(b.n + 15) / 16, 32, 0, st>>>(b);
-    return true;
-  }
-  return false;
-}
-
 template <int L, int OP>
 __global__ void __launch_bounds__(256) finish_kernel(SaberBatch b) {
+  next_may_start();
+  wait_predecessor();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < b.n) sdev::finish_inst<L, OP>(inst_of<L>(b, i, OP));
+}
+
+// The finish on a warp, ten lanes or a pair per state when n is within the thresholds (decaps: one
+// permutation), else on one lane.
+template <int L, int OP>
+cudaError_t launch_finish(const SaberBatch &b, cudaStream_t st, bool follows) {
+  const Tuning &t = tuning();
+  auto blocks = [&](int per) { return (b.n + per - 1) / per; };
+  if constexpr (OP != OP_DEC) {
+    if (b.n <= t.saber_finish_warp_max) return launch_next(follows, finish_multi_kernel<L, OP, 1>, b.n, 32, 0, st, b);
+    if (b.n <= t.saber_finish_five_max) return launch_next(follows, finish_chain_kernel<L, OP>, blocks(3), 64, 0, st, b);
+    if (b.n / 2 <= t.saber_pair_max)  // one sponge per instance, the prologue has two
+      return launch_next(follows, finish_multi_kernel<L, OP, 2>, blocks(16), 32, 0, st, b);
+  }
+  return launch_next(follows, finish_kernel<L, OP>, blocks(t.thread_block), t.thread_block, 0, st, b);
 }
 
 __host__ __device__ constexpr int op_of(int mode) {
@@ -115,6 +194,8 @@ __host__ __device__ constexpr int op_of(int mode) {
 
 template <int L, int MODE, bool I32>
 __global__ void __launch_bounds__(256) product_dp4a_kernel(SaberBatch b) {
+  next_may_start();
+  wait_predecessor();
   extern __shared__ __align__(1024) uint8_t sm[];
   sdev::product_dp4a_cta<L, MODE, I32>(inst_of<L>(b, blockIdx.x, op_of(MODE)), sm, b.sliced != 0);
 }
@@ -122,6 +203,7 @@ __global__ void __launch_bounds__(256) product_dp4a_kernel(SaberBatch b) {
 template <int L, int MODE>
 __global__ void __launch_bounds__(256) product_tc_kernel(SaberBatch b) {
   using Y = TL<L>;
+  next_may_start();
   extern __shared__ __align__(1024) uint8_t sm[];
   uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + Y::TSLOT);
   if (threadIdx.x < 32) {
@@ -132,6 +214,7 @@ __global__ void __launch_bounds__(256) product_tc_kernel(SaberBatch b) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *tslot;
+  wait_predecessor();
   sdev::product_tc_cta<L, MODE>(inst_of<L>(b, blockIdx.x, op_of(MODE)), sm, tbase, b.err, b.sliced != 0);
   tc_fence_before();
   __syncthreads();
@@ -154,6 +237,7 @@ constexpr int kProductCtas = L == 4 ? 4 : 6;
 template <int L, int MODE>
 __global__ void __launch_bounds__(256, kProductCtas<L>) product_tc_persistent_kernel(SaberBatch b) {
   using Y = TL<L>;
+  next_may_start();
   extern __shared__ __align__(1024) uint8_t sm[];
   uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + Y::TSLOT);
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Y::BAR);
@@ -169,6 +253,7 @@ __global__ void __launch_bounds__(256, kProductCtas<L>) product_tc_persistent_ke
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *tslot;
+  wait_predecessor();
   constexpr int op = op_of(MODE);
   sdev::OperandPrefetch<L, MODE> pf;
   int i = blockIdx.x;
@@ -197,7 +282,7 @@ cudaError_t prep(K kernel, int bytes) {
 }
 
 template <int L, int MODE>
-cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st) {
+cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st, bool follows) {
   using Y = PL<L>;
   cudaError_t e;
   if (form == FORM_TC) {
@@ -219,21 +304,20 @@ cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st) {
         sms = m > 0 ? m : 1;
       }
       const int grid = std::min(b.n, sms * std::min(per_sm, kProductCtas<L>));
-      product_tc_persistent_kernel<L, MODE><<<grid, 256, bytes, st>>>(b);
+      return launch_next(follows, product_tc_persistent_kernel<L, MODE>, grid, 256, bytes, st, b);
     } else {
       if ((e = prep(product_tc_kernel<L, MODE>, bytes)) != cudaSuccess) return e;
-      product_tc_kernel<L, MODE><<<b.n, 256, bytes, st>>>(b);
+      return launch_next(follows, product_tc_kernel<L, MODE>, b.n, 256, bytes, st, b);
     }
   } else if (form == FORM_INT32) {
     constexpr int bytes = Y::DP4A_TOTAL;
     if ((e = prep(product_dp4a_kernel<L, MODE, true>, bytes)) != cudaSuccess) return e;
-    product_dp4a_kernel<L, MODE, true><<<b.n, 256, bytes, st>>>(b);
+    return launch_next(follows, product_dp4a_kernel<L, MODE, true>, b.n, 256, bytes, st, b);
   } else {
     constexpr int bytes = Y::DP4A_TOTAL;
     if ((e = prep(product_dp4a_kernel<L, MODE, false>, bytes)) != cudaSuccess) return e;
-    product_dp4a_kernel<L, MODE, false><<<b.n, 256, bytes, st>>>(b);
+    return launch_next(follows, product_dp4a_kernel<L, MODE, false>, b.n, 256, bytes, st, b);
   }
-  return cudaGetLastError();
 }
 
 inline void mark(const SaberBatch &b, cudaStream_t st) {
@@ -243,26 +327,24 @@ inline void mark(const SaberBatch &b, cudaStream_t st) {
 template <int L>
 cudaError_t run(const SaberBatch &batch, int op, int form, cudaStream_t st) {
   SaberBatch b = batch;
-  const int lanes = prologue_lanes(b.n);
-  b.sliced = lanes == 10 || lanes == 2;
-  const int tb = tuning().thread_block;
-  const int fb = (b.n + tb - 1) / tb;
+  b.sliced = prologue_lanes(b.n) == 2;
+  const bool next = b.timer == nullptr && b.n <= kFollowMax;  // stages are timed one after the other
   cudaError_t e;
   mark(b, st);
   switch (op) {
     case OP_KEYPAIR:
-      launch_prologue<L, OP_KEYPAIR>(b, st);
+      if ((e = launch_prologue<L, OP_KEYPAIR>(b, st, false)) != cudaSuccess) return e;
       mark(b, st);
-      if ((e = launch_product<L, sdev::PM_KEYPAIR>(b, form, st)) != cudaSuccess) return e;
+      if ((e = launch_product<L, sdev::PM_KEYPAIR>(b, form, st, next)) != cudaSuccess) return e;
       mark(b, st);
-      if (!launch_finish_multi<L, OP_KEYPAIR>(b, st)) finish_kernel<L, OP_KEYPAIR><<<fb, tb, 0, st>>>(b);
+      if ((e = launch_finish<L, OP_KEYPAIR>(b, st, next)) != cudaSuccess) return e;
       break;
     case OP_ENC:
-      launch_prologue<L, OP_ENC>(b, st);
+      if ((e = launch_prologue<L, OP_ENC>(b, st, false)) != cudaSuccess) return e;
       mark(b, st);
-      if ((e = launch_product<L, sdev::PM_ENC>(b, form, st)) != cudaSuccess) return e;
+      if ((e = launch_product<L, sdev::PM_ENC>(b, form, st, next)) != cudaSuccess) return e;
       mark(b, st);
-      if (!launch_finish_multi<L, OP_ENC>(b, st)) finish_kernel<L, OP_ENC><<<fb, tb, 0, st>>>(b);
+      if ((e = launch_finish<L, OP_ENC>(b, st, next)) != cudaSuccess) return e;
       break;
     default:
       if (b.aux && !b.timer && matrix_beside_inner<L>(b.n)) {
@@ -270,20 +352,21 @@ cudaError_t run(const SaberBatch &batch, int op, int form, cudaStream_t st) {
         // hash chain that follows it.
         if ((e = cudaEventRecord(b.fork, st)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(b.aux, b.fork, 0)) != cudaSuccess) return e;
-        launch_prologue<L, OP_DEC>(b, b.aux, 1, 1);
+        if ((e = launch_prologue<L, OP_DEC>(b, b.aux, false, 1, 1)) != cudaSuccess) return e;
         if ((e = cudaEventRecord(b.join, b.aux)) != cudaSuccess) return e;
-        if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st)) != cudaSuccess) return e;
-        launch_prologue<L, OP_DEC>(b, st, 0, 1);
+        if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st, false)) != cudaSuccess) return e;
+        if ((e = launch_prologue<L, OP_DEC>(b, st, next, 0, 1)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(st, b.join, 0)) != cudaSuccess) return e;
+        if ((e = launch_product<L, sdev::PM_DEC_CMP>(b, form, st, false)) != cudaSuccess) return e;
       } else {
-        if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st)) != cudaSuccess) return e;
+        if ((e = launch_product<L, sdev::PM_DEC_INNER>(b, form, st, false)) != cudaSuccess) return e;
         mark(b, st);
-        launch_prologue<L, OP_DEC>(b, st);
+        if ((e = launch_prologue<L, OP_DEC>(b, st, next)) != cudaSuccess) return e;
+        mark(b, st);
+        if ((e = launch_product<L, sdev::PM_DEC_CMP>(b, form, st, next)) != cudaSuccess) return e;
       }
       mark(b, st);
-      if ((e = launch_product<L, sdev::PM_DEC_CMP>(b, form, st)) != cudaSuccess) return e;
-      mark(b, st);
-      finish_kernel<L, OP_DEC><<<fb, tb, 0, st>>>(b);
+      if ((e = launch_finish<L, OP_DEC>(b, st, next)) != cudaSuccess) return e;
       break;
   }
   mark(b, st);
