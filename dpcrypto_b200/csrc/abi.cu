@@ -222,14 +222,23 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
     }
   }
   const size_t base = arena_need(scheme, op, chunk, !dev);
-  // FrodoKEM on the tensor cores: operand tiles for A generated ahead, as far as the budget
-  // leaves room (none at all is a valid answer).
+  // FrodoKEM on the tensor cores: operand tiles for A generated ahead, as far as the
+  // budget leaves room; none at all is a valid answer, and the one when the device has no memory for
+  // them.  A profiled batch above the size that is generated whole takes none, so that its stages are timed apart.
   const bool frodo_tc = scheme <= DPKEM_FRODO976AES && form == DPKEM_FORM_TC;
   size_t tile_cap = 0;
-  if (frodo_tc && c->budget / npipe > base + kAlign)
-    tile_cap = (size_t)frodo_ahead_count((int)chunk, (c->budget / npipe - base - kAlign) / frodo_ahead_bytes());
-  const size_t per_pipe = up(base + tile_cap * frodo_ahead_bytes());
+  if (frodo_tc && c->budget / npipe > base + kAlign) {
+    const size_t room = (c->budget - (base + kAlign) * npipe) / npipe / frodo_ahead_bytes();
+    tile_cap = (size_t)frodo_ahead_count((int)chunk, room);
+    if (c->profile && tile_cap < chunk) tile_cap = 0;
+  }
+  size_t per_pipe = up(base + tile_cap * frodo_ahead_bytes());
   int rc = ensure_arena(c, per_pipe * npipe);
+  if (rc == DPKEM_ENOMEM && tile_cap) {
+    tile_cap = 0;
+    per_pipe = up(base);
+    rc = ensure_arena(c, per_pipe * npipe);
+  }
   if (rc) return rc;
   cudaError_t e = cudaStreamWaitEvent(st, c->last, 0);
   if (e != cudaSuccess) return cuda_status(e);

@@ -189,16 +189,25 @@ int task_size(int scheme, int kind) {
 // Whether a thread-level stage of a group of `count` requests runs as warp tasks (a warp
 // per instance), and the instances per task either way.
 bool warp_tasks(int kind, size_t count) { return kind != K_CTA && count <= (size_t)tuning().mixed_warp_max; }
-// FrodoKEM sponges run as chain tasks (unless the knob asks for warp tasks).  ms for a batch of one
-// operation on threads / chain tasks: encaps 2,048 requests 10.9 / 8.6, 4,096 18.2 / 16.7, 8,192 32.7 /
-// 32.7; the four-scheme mix of 512 4.6 / 1.6, of 4,096 7.4 / 4.8.
-bool chain_tasks(int scheme, int op, int stage, size_t count) {
-  return chain_stage(scheme, op, stage) && !warp_tasks(kind_of(scheme, op, stage), count);
+// FrodoKEM sponges run as chain tasks, unless the knob asks for warp tasks, or the group is large and the
+// mix has Saber requests enough (`filled`: more than half) to fill the slots that the few thread tasks
+// leave: then the chain tasks' slots cost more than the shorter chains gain.  ms on thread / chain tasks:
+// encaps alone 2,048 requests 10.9 / 8.6, 4,096 18.2 / 16.7, 8,192 32.7 / 32.7; four-scheme mix of 512
+// 4.6 / 1.6, 4,096 7.4 / 4.8, 12,000 (a thousand per FrodoKEM group) 13.8 / 13.1, 16,384 16.4 / 17.1.
+constexpr size_t kChainGroup = 1152;
+bool chain_tasks(int scheme, int op, int stage, size_t count, bool filled) {
+  return chain_stage(scheme, op, stage) && (count <= kChainGroup || !filled) &&
+         !warp_tasks(kind_of(scheme, op, stage), count);
 }
-int task_per(int scheme, int op, int stage, size_t count) {
+bool saber_fills(const Req *reqs, size_t n) {
+  size_t saber = 0;
+  for (size_t i = 0; i < n; i++) saber += reqs[i].scheme > 1;
+  return 2 * saber > n;
+}
+int task_per(int scheme, int op, int stage, size_t count, bool filled) {
   const int kind = kind_of(scheme, op, stage);
   if (kind == K_CTA) return 1;
-  if (chain_tasks(scheme, op, stage, count)) return chain_per(op, stage);
+  if (chain_tasks(scheme, op, stage, count, filled)) return chain_per(op, stage);
   if (warp_tasks(kind, count)) return kind == K_THREAD2 ? 4 : 8;
   return task_size(scheme, kind);
 }
@@ -206,6 +215,7 @@ int task_per(int scheme, int op, int stage, size_t count) {
 // Bytes of device memory a plan for these requests needs (tables + scratch records).
 size_t plan_bytes(const Req *reqs, size_t n, size_t *ntasks_out) {
   size_t scr = 0, ntasks = 0, nidx = 0;
+  const bool filled = saber_fills(reqs, n);
   size_t counts[5][3] = {};
   for (size_t i = 0; i < n; i++) {
     scr += reqs[i].scheme <= 1 ? kFrodoRec : saber_rec_bytes(reqs[i].scheme);
@@ -216,7 +226,7 @@ size_t plan_bytes(const Req *reqs, size_t n, size_t *ntasks_out) {
       const size_t c = counts[s][op];
       if (!c) continue;
       for (int st = 0; st < nstages(s, op); st++) {
-        const size_t per = (size_t)task_per(s, op, st, c);
+        const size_t per = (size_t)task_per(s, op, st, c, filled);
         ntasks += (c + per - 1) / per;
         nidx += c;
       }
@@ -277,6 +287,7 @@ cudaError_t plan_build(const Req *reqs, size_t n, int form, int slots, uint8_t *
     }
     off += r.scheme <= 1 ? kFrodoRec : saber_rec_bytes(r.scheme);
   }
+  const bool filled = saber_fills(reqs, n);
   // Tasks per group and stage; dependencies on the previous stage's tasks are id ranges.
   std::vector<HostTask> ht;
   ht.reserve(ntasks);
@@ -290,8 +301,8 @@ cudaError_t plan_build(const Req *reqs, size_t n, int form, int slots, uint8_t *
     owner.assign(R.size(), -1);
     for (int stg = 0; stg < nstages(scheme, op); stg++) {
       const int kind = kind_of(scheme, op, stg);
-      const int per = task_per(scheme, op, stg, R.size());
-      const bool chain = chain_tasks(scheme, op, stg, R.size()), warp = !chain && warp_tasks(kind, R.size());
+      const int per = task_per(scheme, op, stg, R.size(), filled);
+      const bool chain = chain_tasks(scheme, op, stg, R.size(), filled), warp = !chain && warp_tasks(kind, R.size());
       const uint32_t base = (uint32_t)nid;
       std::memcpy(idx + nid, R.data(), R.size() * 4);
       nid += R.size();
