@@ -35,6 +35,27 @@ __host__ __device__ constexpr Params params(int level) {
 }
 }  // namespace saber
 
+inline int device_sms() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0, m = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
+    sms = m > 0 ? m : 1;
+  }
+  return sms;
+}
+// For kernels whose warps have unlike roles.  A block's warp w runs on SM sub-partition (its first warp
+// slot + w) mod 4, so with fixed roles the long ones of an SM's blocks pile up on the same
+// sub-partitions; this tells a block (all its threads) whether to exchange them: every other four slots.
+__device__ __forceinline__ bool exchange_roles() {
+  if (gridDim.x <= 128) return false;  // a block an SM
+  __shared__ uint32_t slot;
+  if (threadIdx.x == 0) asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+  __syncthreads();
+  return (slot >> 2) & 1;
+}
+
 enum Op : int { OP_KEYPAIR = 0, OP_ENC = 1, OP_DEC = 2 };
 
 // Runtime tuning knobs (set through dpkem_set_tuning; chosen by dpcrypto_b200/autotune.py).
@@ -48,7 +69,7 @@ struct Tuning {
   int mixed_warp_max = 0;
   int pipe_chunks = 4;          // chunks (one stream each) of a pipelined host-mode batch, <= 16
   int pipe_priority = 1;        // 1: chunk streams get descending priorities (earlier chunks finish first)
-  int saber_pair_max = 6144;    // largest Saber batch whose prologue runs on lane pairs (0: never; finish: twice that)
+  int saber_pair_max = 6144;    // largest Saber batch whose sponges run on lane pairs (0: never)
   int saber_warp_max = 512;     // largest Saber batch whose prologue sponges run on a warp per state (0: never)
   int saber_finish_warp_max = 1024;  // the same for the encaps / keypair finish
   // (the *_five_max names are from a layout of five lanes; it is ten now, keccak10.cuh)

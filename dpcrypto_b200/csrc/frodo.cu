@@ -308,17 +308,6 @@ FrodoBatch rest_of(const FrodoBatch &b, int first, int op) {
   return r;
 }
 
-int sm_count() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0, m = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
-    sms = m > 0 ? m : 1;
-  }
-  return sms;
-}
-
 // Chain warps of a front block on ten lanes: four (one per SM sub-partition, 2.05 us per
 // permutation) while the chains outlast the rows, else eight (2.5 us, half the SMs): 2.8 us of the
 // whole chip per instance's rows against the chain's steps.  Measured, n = 128 / 256: encaps 4
@@ -332,8 +321,8 @@ cudaError_t launch_front_g(const FrodoBatch &b, cudaStream_t st) {
   constexpr int steps = STAGE == ahead::F_KEYPAIR ? (HALVE ? 115 : 230) : STAGE == ahead::F_ENC && !HALVE ? 348 : 232;
   const int warps = blocks_for(b.n, spw), cw = NS == 10 ? chain_warps(b.ahead, steps) : 4, chain = blocks_for(warps, cw);
   const int absorb = STAGE == ahead::F_DEC ? (NS == 10 ? blocks_for(b.n, 16 * ahead::kAbsorbWarps) : blocks_for(warps, ahead::kFrontWarps)) : 0;
-  const int early = std::max(0, sm_count() - chain - absorb);
-  const int rows = std::min(sm_count(), std::max(1, ahead::WarpRows<G>::tasks(b.ahead)));
+  const int early = std::max(0, device_sms() - chain - absorb);
+  const int rows = std::min(device_sms(), std::max(1, ahead::WarpRows<G>::tasks(b.ahead)));
   if ((e = set_smem(ahead::front_kernel<STAGE, NS, HALVE, G>, ahead::kFrontSmem)) != cudaSuccess) return e;
   ahead::front_kernel<STAGE, NS, HALVE, G>
       <<<chain + absorb + rows, 32 * ahead::kFrontWarps, ahead::kFrontSmem, st>>>(b, cw, chain, absorb, std::min(early, rows));
@@ -413,7 +402,7 @@ size_t frodo_ahead_bytes() { return ahead::A_BYTES; }
 constexpr int kAheadAll = 1024;
 
 int frodo_ahead_count(int n, size_t cap) {
-  const int wave = 2 * sm_count(), m = n <= kAheadAll ? n : wave + n % wave;
+  const int wave = 2 * device_sms(), m = n <= kAheadAll ? n : wave + n % wave;
   return (int)std::min<size_t>(m, cap);
 }
 

@@ -240,14 +240,15 @@ __global__ void __launch_bounds__(32 * kFrontWarps, 1) front_kernel(FrodoBatch b
 }
 
 // The chains alone, for batches whose A needs no generating (one key) or runs in another form: two
-// chain and two helper warps a block (small blocks spread evenly over the SMs; odd blocks hold the
-// helpers first, so every sub-partition gets both), decaps' absorb blocks after them.
+// chain and two helper warps a block (small blocks spread evenly over the SMs; every other wave of
+// blocks holds the helpers first, so every sub-partition gets both), decaps' absorb blocks after them.
 template <int ROLE>
 __global__ void __launch_bounds__(128, 6) chains_kernel(FrodoBatch b, int chain_blocks) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, block = blockIdx.x;
+  const bool swap = exchange_roles();
   if (block < chain_blocks) {
-    chain_block<ROLE, false, true>(b, block, 2, (warp + 2 * (block & 1)) & 3, smem);
+    chain_block<ROLE, false, true>(b, block, 2, (warp + (swap ? 2 : 0)) & 3, smem);
     return;
   }
   if constexpr (ROLE == R_DEC) absorb_warp(b, (block - chain_blocks) * kAbsorbWarps + warp);

@@ -42,13 +42,21 @@ cudaError_t launch_next(bool follows, void (*kernel)(P...), int grid, int block,
 // Prologue kernels: role 0 is the hash chain and GenSecret, role 1 GenMatrix.  A launch runs both, a
 // warp each (roles = 2, first = 0), or the one `first` names.
 //
+// The role (of two) of this warp: GenMatrix's chain is the longer, so the warps that share a sub-partition
+// must not all run it.  us with fixed roles / exchanged: pairs at 8,192 (l = 3) 145 / 116, one lane at
+// 16,384 (l = 2 / 3 / 4) 112 / 84, 229 / 192, 390 / 290.
+__device__ __forceinline__ int role_warp() {
+  const int w = threadIdx.x >> 5;
+  return blockDim.x == 64 && exchange_roles() ? 1 - w : w;
+}
+
 // One lane per state: 32 instances per block.
 template <int L, int OP>
 __global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b, int first) {
   next_may_start();
   wait_predecessor();
-  const int i = blockIdx.x * 32 + (threadIdx.x & 31);
-  if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), first + (threadIdx.x >> 5));
+  const int i = blockIdx.x * 32 + (threadIdx.x & 31), w = role_warp();
+  if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), first + w);
 }
 
 // Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 10: ten lanes, three
@@ -62,7 +70,7 @@ __global__ void __launch_bounds__(64) prologue_multi_kernel(SaberBatch b, int fi
   wait_predecessor();
   using S = msp::Multi<NS>;
   __shared__ __align__(16) uint8_t xbuf[2 * (S::SMEM_PER_WARP > 0 ? S::SMEM_PER_WARP : 16)];
-  const int w = threadIdx.x >> 5;
+  const int w = role_warp();
   const S s(xbuf + w * S::SMEM_PER_WARP);
   const int g = s.state(), i = blockIdx.x * S::STATES_PER_WARP + g;
   const bool live = g < S::STATES_PER_WARP && i < b.n;
@@ -70,8 +78,7 @@ __global__ void __launch_bounds__(64) prologue_multi_kernel(SaberBatch b, int fi
 }
 
 // Ten lanes per state on chain and helper warps (saber_chain.cuh), three instances per block: the
-// chains of the roles, then their helpers; odd blocks the other way round, so that every SM
-// sub-partition gets both.
+// chains of the roles, then their helpers, exchanged from wave to wave.
 template <int L, int OP>
 __global__ void __launch_bounds__(128) prologue_chain_kernel(SaberBatch b, int first_role, int roles) {
   next_may_start();
@@ -79,7 +86,8 @@ __global__ void __launch_bounds__(128) prologue_chain_kernel(SaberBatch b, int f
   using namespace schain;
   __shared__ Exchange x[2];
   __shared__ __align__(16) uint8_t xbuf[2][k10::kSmemPerWarp];
-  const int warps = 2 * roles, warp = ((threadIdx.x >> 5) + roles * (blockIdx.x & 1)) & (warps - 1);
+  const bool swap = exchange_roles();
+  const int warps = 2 * roles, warp = ((threadIdx.x >> 5) + (swap ? roles : 0)) & (warps - 1);
   const int w = warp & (roles - 1), role = first_role + w, first = 3 * blockIdx.x;
   if (warp < roles) {
     constexpr Program m = Matrix<L, OP>::prog, s = Secret<L, OP>::prog;
@@ -100,7 +108,7 @@ __global__ void __launch_bounds__(64) finish_chain_kernel(SaberBatch b) {
   using namespace schain;
   __shared__ Exchange x;
   __shared__ __align__(16) uint8_t xbuf[k10::kSmemPerWarp];
-  const int warp = ((threadIdx.x >> 5) + blockIdx.x) & 1, lane = threadIdx.x & 31, first = 3 * blockIdx.x;
+  const int warp = (threadIdx.x >> 5) ^ (exchange_roles() ? 1 : 0), lane = threadIdx.x & 31, first = 3 * blockIdx.x;
   if (warp == 0) {
     constexpr Program p = Finish<L, OP>::prog;
     chain_warp(p, x, xbuf, 0);
@@ -182,8 +190,7 @@ cudaError_t launch_finish(const SaberBatch &b, cudaStream_t st, bool follows) {
   if constexpr (OP != OP_DEC) {
     if (b.n <= t.saber_finish_warp_max) return launch_next(follows, finish_multi_kernel<L, OP, 1>, b.n, 32, 0, st, b);
     if (b.n <= t.saber_finish_five_max) return launch_next(follows, finish_chain_kernel<L, OP>, blocks(3), 64, 0, st, b);
-    if (b.n / 2 <= t.saber_pair_max)  // one sponge per instance, the prologue has two
-      return launch_next(follows, finish_multi_kernel<L, OP, 2>, blocks(16), 32, 0, st, b);
+    if (b.n <= t.saber_pair_max) return launch_next(follows, finish_multi_kernel<L, OP, 2>, blocks(16), 32, 0, st, b);
   }
   return launch_next(follows, finish_kernel<L, OP>, blocks(t.thread_block), t.thread_block, 0, st, b);
 }
@@ -292,18 +299,15 @@ cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st, bool 
       // persistent: per_sm CTAs per SM, several instances each.  The CTAs never wait on one
       // another, so a grid larger than what is resident only queues; TMEM (32 columns per
       // CTA) fits 16 CTAs per SM.
-      static int sms = 0;  // per process and instantiation
-      if (!sms) {
-        if ((e = prep(product_tc_persistent_kernel<L, MODE>, bytes)) != cudaSuccess) return e;
+      if ((e = prep(product_tc_persistent_kernel<L, MODE>, bytes)) != cudaSuccess) return e;
+      static bool carved = false;  // per process and instantiation
+      if (!carved) {
         if ((e = cudaFuncSetAttribute(product_tc_persistent_kernel<L, MODE>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess)
           return e;
-        int dev = 0, m = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        sms = m > 0 ? m : 1;
+        carved = true;
       }
-      const int grid = std::min(b.n, sms * std::min(per_sm, kProductCtas<L>));
+      const int grid = std::min(b.n, device_sms() * std::min(per_sm, kProductCtas<L>));
       return launch_next(follows, product_tc_persistent_kernel<L, MODE>, grid, 256, bytes, st, b);
     } else {
       if ((e = prep(product_tc_kernel<L, MODE>, bytes)) != cudaSuccess) return e;

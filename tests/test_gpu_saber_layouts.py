@@ -55,7 +55,7 @@ def test_layouts(engine, oracle, scheme, layout):
         _run(engine, oracle, scheme, 101)  # partial warps of ten lanes (3), pairs (16), one lane (32)
 
 
-@pytest.mark.parametrize("scheme,n", [(d.SABER, 300), (d.SABER, 301), (d.FIRESABER, 1793), (d.SABER, 4737),
+@pytest.mark.parametrize("scheme,n", [(d.SABER, 300), (d.SABER, 301), (d.FIRESABER, 1793), (d.SABER, 4737), (d.SABER, 9472),
                                       (d.LIGHTSABER, 9473), (d.FIRESABER, 12000)])
 def test_rule_edges(engine, oracle, scheme, n):
     _run(engine, oracle, scheme, n)
