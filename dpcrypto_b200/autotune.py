@@ -12,7 +12,7 @@ Knobs:
   pipe_priority      chunk streams with descending priorities (earlier chunks finish first)
   lanes per state    per sponge stage (Saber prologue, Saber encaps finish, Frodo prologue,
                      Frodo shared-secret hash) and batch size: a warp per state
-                     (*_warp_max), five lanes (*_five_max), a lane pair (saber_pair_max,
+                     (*_warp_max), ten lanes (*_five_max), a lane pair (saber_pair_max,
                      Saber only) or one lane.  Each layout is forced in turn at 64-16k
                      instances (Frodo 64-8k) and timed with the stage timer; a layout covers batches up
                      to the largest swept size at which it was the fastest
@@ -206,7 +206,7 @@ def _child(u: int) -> dict:
     return res
 
 # Lanes per state of each sponge stage, by batch size.  Every layout is forced in turn with
-# the thresholds of the stage (a warp per state first, then five lanes, then the pair, else
+# the thresholds of the stage (a warp per state first, then ten lanes, then the pair, else
 # one lane); the stage's device time comes from the stage timer of an encaps + decaps.
 BIG = 1 << 30
 SABER_SIZES = (64, 256, 512, 1024, 2048, 4096, 8192, 16384)

@@ -1,5 +1,6 @@
-// Keccak-f[1600] with one state spread over five lanes of a warp, for sponge chains on the
-// critical path of a latency-bound stage.
+// Keccak-f[1600] with one state spread over five lanes of a warp: one of the layouts that
+// dpkem_keccak_f1600_lanes and dpkem_probe_keccak_chain compare.  The stages run keccak10.cuh instead
+// (1,024 states: 2.11 us a permutation against 3.38 here).
 //
 // A warp holds six states: lanes 5g .. 5g+4 form group g (lanes 30 and 31 run along in a
 // seventh, partial group whose results are never stored).  Thread t of a group owns five of
@@ -19,9 +20,7 @@
 // That is 48 integer instructions, 14 shuffles and 10 shared-memory accesses per thread and
 // round, against 180 integer instructions for a whole state on one thread: the dependent
 // chain of a sponge gets about 2.5x fewer instructions per thread, at the price of more
-// instructions per state in total.  It pays where a stage leaves SM sub-partitions idle
-// (small batches, the serial sponges of a prologue) and loses where the integer pipe is
-// already saturated, so lanes per state is a tuning knob of each stage.
+// instructions per state in total.
 //
 // Every lane of the warp must execute the shuffles and the warp syncs: callers keep whole
 // warps in step and predicate only global-memory accesses (live = false for a group without
@@ -119,88 +118,6 @@ __device__ __forceinline__ void round5(uint2 (&a)[5], const Lanes &k, uint2 rcv)
 __device__ __forceinline__ void f1600(uint2 (&a)[5], const Lanes &k) {
 #pragma unroll 1
   for (int r = 0; r < 24; r++) round5(a, k, c_keccak_rc[r]);
-}
-
-__device__ __forceinline__ void zero(uint2 (&a)[5]) {
-#pragma unroll
-  for (int y = 0; y < 5; y++) a[y] = make_uint2(0u, 0u);
-}
-
-// Lane i (= x + 5y) of the state, broadcast to every thread of the group.
-template <int I>
-__device__ __forceinline__ uint2 get(const uint2 (&a)[5], const Lanes &k) {
-  return shfl(a[I / 5], k.base + I % 5);
-}
-
-// XOR w into lane I (only the owning thread's copy of w matters).
-template <int I>
-__device__ __forceinline__ void xor_lane(uint2 (&a)[5], const Lanes &k, uint2 w) {
-  if (k.t == I % 5) {
-    a[I / 5].x ^= w.x;
-    a[I / 5].y ^= w.y;
-  }
-}
-
-// Absorb whole 8-byte words: word q of the message block goes into lane q.  The owning
-// thread loads its own words (lanes t, t + 5, ...); `len` is a multiple of 8, p 8-byte
-// aligned, `pos` the current fill (multiple of 8).  Returns the new fill.
-template <int RATE>
-__device__ __forceinline__ int absorb_aligned(uint2 (&a)[5], const Lanes &k, int pos, const uint8_t *p, int len,
-                                              bool live) {
-  constexpr int W = RATE / 8;
-  while (len > 0) {
-    const int take = min(len, RATE - pos);
-    const int q0 = pos / 8, nq = take / 8;
-#pragma unroll
-    for (int y = 0; y < 5; y++) {
-      const int q = k.t + 5 * y;  // the lane this slot holds
-      if (q < W && q >= q0 && q < q0 + nq && live) {
-        const uint2 w = ld_lane(p + 8 * (q - q0));
-        a[y].x ^= w.x;
-        a[y].y ^= w.y;
-      }
-    }
-    pos += take;
-    p += take;
-    len -= take;
-    if (pos == RATE) {
-      f1600(a, k);
-      pos = 0;
-    }
-  }
-  return pos;
-}
-
-// Padding (domain byte at `pos`, 0x80 in the last rate byte), then the permutation.
-template <int RATE>
-__device__ __forceinline__ void absorb_finish(uint2 (&a)[5], const Lanes &k, int pos, uint32_t domain) {
-  const int qd = pos / 8, sh = 8 * (pos % 8), ql = RATE / 8 - 1;
-#pragma unroll
-  for (int y = 0; y < 5; y++) {
-    const int q = k.t + 5 * y;
-    if (q == qd) {
-      if (sh < 32) a[y].x ^= domain << sh;
-      else a[y].y ^= domain << (sh - 32);
-    }
-    if (q == ql) a[y].y ^= 0x80000000u;
-  }
-  f1600(a, k);
-}
-
-// Squeeze `len` bytes (a multiple of 8) to dst, permuting between rate blocks; the state
-// must have been finished.  Each thread stores the lanes it owns.
-template <int RATE>
-__device__ __forceinline__ void squeeze(uint2 (&a)[5], const Lanes &k, uint8_t *dst, int len, bool live) {
-  constexpr int W = RATE / 8;
-  for (int off = 0;; off += RATE) {
-#pragma unroll
-    for (int y = 0; y < 5; y++) {
-      const int q = k.t + 5 * y;
-      if (q < W && off + 8 * q < len && live) *reinterpret_cast<uint2 *>(dst + off + 8 * q) = a[y];
-    }
-    if (off + RATE >= len) break;
-    f1600(a, k);
-  }
 }
 
 }  // namespace k5

@@ -3,12 +3,12 @@
 // (mixed.cu) run the same code.
 //
 // Kernel chain per operation:
-//   prologue  (64 threads = 32 instances: warp 0 runs the hash chain and GenSecret's
-//              SHAKE128 (decaps: then SHA3-256 of the input ciphertext), warp 1 runs
-//              GenMatrix's SHAKE128, in parallel; raw XOF bytes go to the scratch arena)
+//   prologue  (two sponges an instance: role 0 the hash chain and GenSecret's SHAKE128, decaps: then
+//              SHA3-256 of the input ciphertext; role 1 GenMatrix's SHAKE128; XOF bytes go to the
+//              scratch arena.  Lanes per state by batch size, saber.cu)
 //   product   (CTA/instance: CBD sampling, 13/10-bit unpacking, the negacyclic
 //              matrix-vector and inner products, rounding, packing / comparison)
-//   finish    (thread/instance: SHA3-256(c) (encaps), final key, or H(pk) for keypair)
+//   finish    (SHA3-256(c) (encaps), final key, or H(pk) for keypair)
 // Decaps runs the product kernel twice: first the inner product v = b'^T s with the
 // secret from sk (-> m'), then the re-encryption in compare mode.
 //
