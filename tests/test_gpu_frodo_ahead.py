@@ -1,7 +1,8 @@
 """FrodoKEM batches whose A is generated ahead of its use (tensor-core form, a key per
 instance): every byte against the dp4a form on every instance and against the CPU oracle on a
 sample, at the sizes where the split of a batch changes (one instance, the columns of a product
-split over one, two and four CTAs, the largest batch generated whole, one past it)."""
+split over one, two and four CTAs, the largest batch generated whole, the largest on ten lanes and
+the largest on lane pairs, each with the size after it)."""
 import os
 
 import numpy as np
@@ -19,8 +20,8 @@ def _sample(n):
 
 
 @pytest.mark.parametrize("scheme,n", [(s, n) for s in (d.FRODO976, d.FRODO976AES)
-                                      for n in (1, 3, 49, 50, 98, 99, 297)] + [(d.FRODO976, 444), (d.FRODO976, 445),
-                                                                               (d.FRODO976, 1100)])
+                                      for n in (1, 3, 49, 50, 98, 99, 297)] +
+                         [(d.FRODO976, n) for n in (444, 445, 1024, 1025, 1100, 4096, 4097, 9472, 9473)])
 def test_ahead_equals_dp4a_and_oracle(engine, oracle, scheme, n):
     kc = torch.empty((n, 64), dtype=torch.uint8, device="cuda")
     ec = torch.empty((n, 24), dtype=torch.uint8, device="cuda")
