@@ -100,6 +100,11 @@ int cuda_status(cudaError_t e) {
   return DPKEM_ECUDA;
 }
 
+std::atomic<int> &open_services(int device) {
+  static std::atomic<int> open[64];
+  return open[device & 63];
+}
+
 cudaError_t persistent_grid(const dpkem_ctx *c, int *grid) {
   const cudaError_t e = mixed::kernel_setup(grid);
   if (e == cudaSuccess && c->max_ctas > 0) *grid = std::min(*grid, c->max_ctas);
@@ -225,7 +230,10 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
   // FrodoKEM on the tensor cores: operand tiles for A generated ahead, as far as the
   // budget leaves room; none at all is a valid answer, and the one when the device has no memory for
   // them.  A profiled batch above the size that is generated whole takes none, so that its stages are timed apart.
-  const bool frodo_tc = scheme <= DPKEM_FRODO976AES && form == DPKEM_FORM_TC;
+  // Nor does a batch beside an open service: a front block (512 threads, 89-128 registers, 120 KB) does not fit
+  // on an SM that holds a CTA of the service (256 x 128 registers, 107 KB) and would wait until the
+  // service's launch ends; the kernels of the path without tiles fit beside one.
+  const bool frodo_tc = scheme <= DPKEM_FRODO976AES && form == DPKEM_FORM_TC && open_services(c->device).load() == 0;
   size_t tile_cap = 0;
   if (frodo_tc && c->budget / npipe > base + kAlign) {
     const size_t room = (c->budget - (base + kAlign) * npipe) / npipe / frodo_ahead_bytes();

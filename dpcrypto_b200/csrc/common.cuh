@@ -166,6 +166,9 @@ size_t frodo_gemm_ab_bytes();
 // them, and that scratch per instance.
 int frodo_ahead_count(int n, size_t cap);
 size_t frodo_ahead_bytes();
+// Loads the kernels of the tensor-core form without operand tiles, which batches run beside an open
+// service (dpkem_service_open): a first launch there would wait until the service's launch ends.
+cudaError_t frodo_load_untiled();
 size_t frodo_gemm_s_bytes(size_t n);
 cudaError_t frodo_pk_digest(const uint8_t *pk, uint8_t *out, cudaStream_t st);
 

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
@@ -49,6 +50,8 @@ int set_status(int s);                      // records the calling thread's last
 bool scheme_sizes(int scheme, Sizes *z);    // object sizes of a scheme; false if unknown
 int ensure_arena(dpkem_ctx *c, size_t bytes);  // grows the context's device arena
 int cuda_status(cudaError_t e);             // DPKEM_OK or DPKEM_ECUDA (clears the error)
+// Services open on a device (serve.cu): their launches hold CTAs for as long as requests come.
+std::atomic<int> &open_services(int device);
 // Grid of this context's persistent launches: the device's resident CTAs, capped by max_ctas.
 cudaError_t persistent_grid(const dpkem_ctx *c, int *grid);
 // Pinned stage j of at least `bytes`, once its previous upload has run (nullptr if it

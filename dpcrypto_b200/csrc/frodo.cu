@@ -383,6 +383,32 @@ cudaError_t frodo_expand_a(int aes, const uint8_t *pk, uint16_t *amat, cudaStrea
   return cudaGetLastError();
 }
 
+// The driver loads a kernel's code at its first launch, for which it waits until the device is idle.
+cudaError_t frodo_load_untiled() {
+  const void *const kernels[] = {
+      (const void *)ahead::kp_seed_kernel, (const void *)ahead::chains_kernel<ahead::R_KEYPAIR>,
+      (const void *)ahead::chains_kernel<ahead::R_ENC>, (const void *)ahead::chains_kernel<ahead::R_DEC>,
+      (const void *)stage_multi_kernel<0, 2>, (const void *)stage_multi_kernel<2, 2>,
+      (const void *)kp_prologue_kernel<OP_KEYPAIR>, (const void *)prologue_kernel<OP_ENC>,
+      (const void *)dec_prologue_kernel, (const void *)dec_w_kernel,
+      (const void *)kp_as_tc_kernel<fdev::KPT_NST, fdev::ShakeRows>, (const void *)kp_as_tc_kernel<1, fdev::AesRowsFull>,
+      (const void *)sa_tc_kernel<OP_ENC, kTcStages, fdev::ShakeRows>,
+      (const void *)sa_tc_kernel<OP_DEC, kTcStages, fdev::ShakeRows>,
+      (const void *)sa_tc_kernel<OP_ENC, 1, fdev::AesRowsFull>, (const void *)sa_tc_kernel<OP_DEC, 1, fdev::AesRowsFull>,
+      (const void *)stage_multi_kernel<1, 1>, (const void *)stage_multi_kernel<1, 10>,
+      (const void *)stage_multi_kernel<1, 2>, (const void *)stage_multi_kernel<3, 1>,
+      (const void *)stage_multi_kernel<3, 10>, (const void *)stage_multi_kernel<3, 2>,
+      (const void *)stage_multi_kernel<4, 1>, (const void *)stage_multi_kernel<4, 10>,
+      (const void *)stage_multi_kernel<4, 2>, (const void *)pk_hash_kernel<OP_KEYPAIR>, (const void *)ss_kernel<OP_ENC>,
+      (const void *)ss_kernel<OP_DEC>};
+  cudaFuncAttributes a;
+  for (const void *k : kernels) {
+    const cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 size_t frodo_gemm_ab_bytes() { return fgemm::AB_BYTES; }
 size_t frodo_gemm_s_bytes(size_t n) { return fgemm::s_bytes((int)n); }
 

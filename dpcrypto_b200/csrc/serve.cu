@@ -624,6 +624,7 @@ int dpkem_service_open(dpkem_ctx *c, int form, const dpkem_service_config *cfg_i
   if (e == cudaSuccess) e = cudaFuncSetAttribute(serve::service_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  mixed::kSmem);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->kst);
+  if (e == cudaSuccess) e = frodo_load_untiled();
   if (e == cudaSuccess) {
     int sms = 0, occ = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
@@ -658,6 +659,7 @@ int dpkem_service_open(dpkem_ctx *c, int form, const dpkem_service_config *cfg_i
       std::memcpy(&hi, cfg.coin_key + 8 * q + 4, 4);
       p.key.w[q] = make_uint2(lo, hi);
     }
+  open_services(c->device)++;
   *out = s;
   return set_status(DPKEM_OK);
 }
@@ -786,6 +788,7 @@ int dpkem_service_close(dpkem_service *s) {
     if (e != cudaSuccess && rc == DPKEM_OK) rc = cuda_status(e);
     if (rc == DPKEM_OK && s->h_map[s->slots]) rc = DPKEM_ETIMEOUT;
   }
+  open_services(s->c->device)--;
   release(s);
   return set_status(rc);
 }
