@@ -17,10 +17,23 @@ using sdev::TL;
 // The stages of a call follow one another at once: each kernel lets the next one's blocks start when
 // all of its own have, and waits for its predecessor's results itself (programmatic dependent launch), so
 // launch latency and a kernel's set-up pass while the predecessor drains.  The first kernel of a call is
-// launched plainly and waits for the whole stream.  Only up to kFollowMax instances: a waiting kernel
+// launched plainly and waits for the whole stream.  Only up to follow_max instances: a waiting kernel
 // that fills the SMs keeps the next call's sponges, or a persistent product's CTAs, off them.  us, plain /
 // following, encaps at l = 3: n = 1 80 / 74, 444 86 / 82, 600 89 / 88, 1,501 112 / 140, 4,096 149 / 202.
-constexpr int kFollowMax = 512;
+// FireSaber's product CTAs, started early, share SMs that the prologue leaves free instead of spreading
+// over all of them, where they are long and the prologue's blocks uneven.  us, plain / following, at l = 4:
+//   tensor-core  encaps 300 125 / 125, 444 128 / 126, 512 128 / 143; keypair 444 129 / 129, 512 130 / 136
+//   dp4a         encaps 100 130 / 127, 200 136 / 140, 300 144 / 170; keypair 148 133 / 131, 256 138 / 150; decaps
+//                300 126 / 122, 512 147 / 145
+//   INT32        encaps 100 144 / 140, 148 144 / 158, 300 181 / 236; keypair 300 176 / 173, 512 195 / 193; decaps
+//                350 190 / 183, 400 188 / 204
+// (l = 3, INT32 encaps: 300 124 / 119, 512 137 / 134).
+template <int L>
+constexpr int follow_max(int op, int form) {
+  if (L < 4) return 512;
+  if (form == FORM_TC) return 444;
+  return op == OP_ENC ? 100 : op == OP_KEYPAIR ? (form == FORM_INT32 ? 512 : 148) : form == FORM_INT32 ? 350 : 512;
+}
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -332,7 +345,7 @@ template <int L>
 cudaError_t run(const SaberBatch &batch, int op, int form, cudaStream_t st) {
   SaberBatch b = batch;
   b.sliced = prologue_lanes(b.n) == 2;
-  const bool next = b.timer == nullptr && b.n <= kFollowMax;  // stages are timed one after the other
+  const bool next = b.timer == nullptr && b.n <= follow_max<L>(op, form);  // stages are timed one after the other
   cudaError_t e;
   mark(b, st);
   switch (op) {
