@@ -141,10 +141,19 @@ __global__ void __launch_bounds__(64) finish_chain_kernel(SaberBatch b) {
 
 // Lanes per state of the prologue's sponges for a batch of n: a warp per state up to
 // saber_warp_max, ten lanes up to saber_five_max (the knob's name is from a layout of five), a
-// pair up to saber_pair_max, else one.
+// pair up to saber_pair_max (LightSaber decaps, whose two chains are the shortest: half of that), else one.
+// us, decaps at l = 2 on pairs / one lane: tensor-core 4,096 105 / 120, 5,000 133 / 129, 8,192 173 / 164;
+// dp4a 4,096 182 / 197, 5,000 228 / 223, 8,192 325 / 315 (l = 3, 9,472 261 / 268; keypair at l = 2 136 / 157).
+template <int L, int OP>
 int prologue_lanes(int n) {
   const Tuning &t = tuning();
-  return n <= t.saber_warp_max ? 25 : n <= t.saber_five_max ? 10 : n <= t.saber_pair_max ? 2 : 1;
+  const int pair_max = L == 2 && OP == OP_DEC ? t.saber_pair_max / 2 : t.saber_pair_max;
+  return n <= t.saber_warp_max ? 25 : n <= t.saber_five_max ? 10 : n <= pair_max ? 2 : 1;
+}
+template <int L>
+int prologue_lanes(int n, int op) {
+  return op == OP_KEYPAIR ? prologue_lanes<L, OP_KEYPAIR>(n) : op == OP_ENC ? prologue_lanes<L, OP_ENC>(n)
+                                                                            : prologue_lanes<L, OP_DEC>(n);
 }
 
 // Whether decaps runs GenMatrix on a second stream beside the inner product and the chain that needs
@@ -155,7 +164,7 @@ int prologue_lanes(int n) {
 // 12,000 413 / 388, 16,384 474 / 448; l = 4: 128 115 / 109, 12,000 669 / 539; l = 2: 128 49 / 51.
 template <int L>
 bool matrix_beside_inner(int n) {
-  const int lanes = prologue_lanes(n);
+  const int lanes = prologue_lanes<L, OP_DEC>(n);
   return L > 2 && ((lanes == 25 && n <= 100) || (lanes == 10 && n <= 300) || (lanes == 1 && n >= 12000));
 }
 
@@ -163,7 +172,7 @@ template <int L, int OP>
 cudaError_t launch_prologue(const SaberBatch &b, cudaStream_t st, bool follows, int first = 0, int roles = 2) {
   auto blocks = [&](int per) { return (b.n + per - 1) / per; };
   const int threads = 32 * roles;
-  switch (prologue_lanes(b.n)) {
+  switch (prologue_lanes<L, OP>(b.n)) {
     case 25: return launch_next(follows, prologue_multi_kernel<L, OP, 1>, b.n, threads, 0, st, b, first);
     case 10: return launch_next(follows, prologue_chain_kernel<L, OP>, blocks(3), 2 * threads, 0, st, b, first, roles);
     case 2: return launch_next(follows, prologue_multi_kernel<L, OP, 2>, blocks(16), threads, 0, st, b, first);
@@ -344,7 +353,7 @@ inline void mark(const SaberBatch &b, cudaStream_t st) {
 template <int L>
 cudaError_t run(const SaberBatch &batch, int op, int form, cudaStream_t st) {
   SaberBatch b = batch;
-  b.sliced = prologue_lanes(b.n) == 2;
+  b.sliced = prologue_lanes<L>(b.n, op) == 2;
   const bool next = b.timer == nullptr && b.n <= follow_max<L>(op, form);  // stages are timed one after the other
   cudaError_t e;
   mark(b, st);

@@ -1,5 +1,5 @@
 """Saber batches on both sides of the rules that depend on level and form: how a call's kernels follow one
-another (FireSaber).  Every byte of all forms against one another and of a sample against the CPU oracle."""
+another (FireSaber), where decaps leave the lane pairs (LightSaber).  Every byte of all forms against one another and of a sample against the CPU oracle."""
 import os
 
 import numpy as np
@@ -42,3 +42,8 @@ def _check(engine, oracle, scheme, n, forms):
 @pytest.mark.parametrize("n", [100, 101, 148, 149, 350, 351, 444, 445, 512, 513])
 def test_following_kernels(engine, oracle, n):
     _check(engine, oracle, d.FIRESABER, n, (d.FORM_TC, d.FORM_DP4A, d.FORM_INT32))
+
+
+@pytest.mark.parametrize("n", [4736, 4737])
+def test_lightsaber_decaps_pairs(engine, oracle, n):
+    _check(engine, oracle, d.LIGHTSABER, n, (d.FORM_TC, d.FORM_DP4A))
