@@ -263,15 +263,17 @@ cudaError_t launch_kp_as(const FrodoBatch &b, int form, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The prologue without A's rows: on chain and helper warps up to frodo_warp_max / frodo_five_max
-// (decaps, whose ciphertext hash shares the SMs, up to two thirds of that), encaps and keypair
-// on pairs up to kPairMax; false above.  us, encaps under one key: n = 4,096 780 (five lanes 1,082),
-// 6,000 995, 8,192 on pairs 1,088, on one lane 1,497; decaps: 512 469 (a warp per state 682), 4,096 932
-// (five lanes 1,665), 5,000 1,448 against 1,470 on one lane.
+// The prologue without A's rows: on chain and helper warps up to frodo_warp_max / frodo_five_max (decaps,
+// whose ciphertext hash shares the SMs, at most to kDecChains), encaps and keypair on pairs up to
+// kPairMax; false above.  us of the whole call under one key, chains / pairs, encaps: n = 4,096 1,508 / 1,719,
+// 6,144 1,782 / 1,832, 7,000 1,903 / 1,853; chains / one lane, decaps: 1,024 655 / 1,544, 4,096 1,121 / 1,662, 4,871 (the
+// blocks that are resident at once end there) 1,327 / 1,696, 5,300 1,387 / 1,706, 5,700 1,609 / 1,721, 6,144
+// 1,816 / 1,738.
+constexpr int kDecChains = 5600;
 template <int ROLE>
 bool launch_prologue(const FrodoBatch &b, cudaStream_t st) {
   const int most = std::max(tuning().frodo_warp_max, tuning().frodo_five_max);
-  if (b.n <= (ROLE == ahead::R_DEC ? most - most / 3 : most)) {
+  if (b.n <= (ROLE == ahead::R_DEC ? std::min(most, kDecChains) : most)) {
     const int chain = blocks_for(b.n, 6), absorb = ROLE == ahead::R_DEC ? blocks_for(b.n, 16 * ahead::kAbsorbWarps) : 0;
     if (ROLE == ahead::R_KEYPAIR) ahead::kp_seed_kernel<<<blocks_for(b.n, 32), 32, 0, st>>>(b);
     ahead::chains_kernel<ROLE><<<chain + absorb, 128, ahead::chain_smem(2), st>>>(b, chain);
