@@ -58,30 +58,34 @@ __device__ __forceinline__ bool exchange_roles() {
 
 enum Op : int { OP_KEYPAIR = 0, OP_ENC = 1, OP_DEC = 2 };
 
-// Runtime tuning knobs (set through dpkem_set_tuning; chosen by dpcrypto_b200/autotune.py).
+// Runtime tuning knobs (set through dpkem_set_tuning).  The defaults, which a C program runs with, are the values
+// chosen in dpcrypto_b200/tuning.json, which the Python package applies when it loads the library.  (The
+// *_five_max names are from a layout of five lanes; it is ten now, keccak10.cuh.)
 struct Tuning {
-  int thread_block = 64;        // block size of the thread-per-instance kernels
-  int mixed_frodo_task = 256;   // instances per Frodo thread-level task in a mixed batch
+  int thread_block = 32;        // block size of the thread-per-instance kernels
+  int mixed_frodo_task = 128;   // instances per Frodo thread-level task in a mixed batch
   int mixed_pair_task = 128;    // instances per two-role prologue task (two threads each)
   int mixed_thread_task = 256;  // instances per other thread-level task
   // groups of up to this many requests run their sponge stages on a warp each (0: never).
   // Off: a planned batch of 32 mixed requests took 12.2 ms with warp tasks, 4.5 ms without
   int mixed_warp_max = 0;
-  int pipe_chunks = 4;          // chunks (one stream each) of a pipelined host-mode batch, <= 16
+  int pipe_chunks = 8;          // chunks (one stream each) of a pipelined host-mode batch, <= 16
   int pipe_priority = 1;        // 1: chunk streams get descending priorities (earlier chunks finish first)
-  int saber_pair_max = 6144;    // largest Saber batch whose sponges run on lane pairs (0: never)
-  int saber_warp_max = 512;     // largest Saber batch whose prologue sponges run on a warp per state (0: never)
-  int saber_finish_warp_max = 1024;  // the same for the encaps / keypair finish
-  // (the *_five_max names are from a layout of five lanes; it is ten now, keccak10.cuh)
-  int saber_five_max = 0;       // largest Saber batch whose prologue sponges run on ten lanes per state (0: never)
-  int saber_finish_five_max = 0;  // the same for the encaps / keypair finish
-  // the larger of frodo_warp_max and frodo_five_max: largest Frodo batch whose prologues run on chain
-  // and helper warps (frodo_ahead.cuh; 0: never)
-  int frodo_warp_max = 1024;
-  int frodo_ss_warp_max = 1024; // the same on a warp per state
-  int frodo_five_max = 0;
-  int frodo_ss_five_max = 0;    // largest Frodo batch whose H(pk) and final hash run on ten lanes per state (0: never)
-  int saber_tc_ctas_per_sm = 0; // persistent Saber tensor-core product CTAs per SM (0: a CTA per instance)
+  // largest Saber batch whose prologue sponges run on a warp per state / ten lanes / a lane pair (0: never)
+  int saber_warp_max = 0;
+  int saber_five_max = 2048;
+  int saber_pair_max = 9472;    // encaps / keypair finish too
+  // the same for the encaps / keypair finish
+  int saber_finish_warp_max = 32;
+  int saber_finish_five_max = 3072;
+  // the larger of the two: largest Frodo batch whose prologues run on chain and helper warps
+  // (frodo_ahead.cuh; 0: never)
+  int frodo_warp_max = 512;
+  int frodo_five_max = 6144;
+  // largest Frodo batch whose H(pk) and final hash run on a warp per state / ten lanes (0: never)
+  int frodo_ss_warp_max = 512;
+  int frodo_ss_five_max = 3072;
+  int saber_tc_ctas_per_sm = 6; // persistent Saber tensor-core product CTAs per SM (0: a CTA per instance)
 };
 Tuning &tuning();
 

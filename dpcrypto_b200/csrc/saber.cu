@@ -22,7 +22,8 @@ using sdev::TL;
 // following, encaps at l = 3: n = 1 80 / 74, 444 86 / 82, 600 89 / 88, 1,501 112 / 140, 4,096 149 / 202.
 // FireSaber's product CTAs, started early, share SMs that the prologue leaves free instead of spreading
 // over all of them, where they are long and the prologue's blocks uneven.  us, plain / following, at l = 4:
-//   tensor-core  encaps 300 125 / 125, 444 128 / 126, 512 128 / 143; keypair 444 129 / 129, 512 130 / 136
+//   tensor-core  encaps 300 125 / 125, 444 128 / 126, 512 128 / 143; keypair 444 129 / 129, 512 130 / 136; decaps
+//                512 117 / 115
 //   dp4a         encaps 100 130 / 127, 200 136 / 140, 300 144 / 170; keypair 148 133 / 131, 256 138 / 150; decaps
 //                300 126 / 122, 512 147 / 145
 //   INT32        encaps 100 144 / 140, 148 144 / 158, 300 181 / 236; keypair 300 176 / 173, 512 195 / 193; decaps
@@ -31,7 +32,7 @@ using sdev::TL;
 template <int L>
 constexpr int follow_max(int op, int form) {
   if (L < 4) return 512;
-  if (form == FORM_TC) return 444;
+  if (form == FORM_TC) return op == OP_DEC ? 512 : 444;
   return op == OP_ENC ? 100 : op == OP_KEYPAIR ? (form == FORM_INT32 ? 512 : 148) : form == FORM_INT32 ? 350 : 512;
 }
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
