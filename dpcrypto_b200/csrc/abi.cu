@@ -73,25 +73,40 @@ size_t chunk_for(dpkem_ctx *c, int scheme, int op, bool host) {
 }
 
 // Growing the arena frees the old one (cudaFree waits for the whole device, other
-// contexts' work included), so growth is geometric (at least 1.5x, within the budget) and
-// callers on a latency path reserve the arena up front (dpkem_ctx_reserve).
-int ensure_arena(dpkem_ctx *c, size_t bytes) {
-  if (bytes <= c->arena_bytes) return DPKEM_OK;
-  if (bytes > c->budget) return DPKEM_ENOMEM;
-  const size_t want = std::min(c->budget, std::max(bytes, c->arena_bytes + c->arena_bytes / 2));
-  if (c->arena) {
-    // c->last follows every launch that used the arena, on whichever stream it ran
-    cudaEventSynchronize(c->last);
-    cudaFree(c->arena);
-    c->arena = nullptr;
-    c->arena_bytes = 0;
-  }
-  if (cudaMalloc(&c->arena, want) != cudaSuccess) {
+// contexts' work included), so growth is geometric and callers on a latency path reserve the arena up front
+// (dpkem_ctx_reserve).
+struct CtxMem final : ArenaMem {
+  dpkem_ctx *c;
+  explicit CtxMem(dpkem_ctx *ctx) : c(ctx) {}
+  void *alloc(size_t bytes) override {
+    void *p = nullptr;
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
     cudaGetLastError();
-    return DPKEM_ENOMEM;
+    return nullptr;
   }
-  c->arena_bytes = want;
-  return DPKEM_OK;
+  void release(void *p) override { cudaFree(p); }
+  void drain() override {  // c->last follows every launch that used the arena, on whichever stream it ran
+    if (cudaEventSynchronize(c->last) != cudaSuccess) cudaGetLastError();
+  }
+};
+
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {  // the legacy stream during another stream's capture
+    cudaGetLastError();
+    return false;
+  }
+  return s != cudaStreamCaptureStatusNone;
+}
+
+int ensure_arena(dpkem_ctx *c, size_t bytes, cudaStream_t st) {
+  if (st && capturing(st)) {
+    if (bytes > c->arena.bytes) return DPKEM_ENOMEM;
+    c->arena.captured();
+    return DPKEM_OK;
+  }
+  CtxMem mem(c);
+  return c->arena.need(bytes, c->budget, mem) ? DPKEM_OK : DPKEM_ENOMEM;
 }
 
 int cuda_status(cudaError_t e) {
@@ -227,26 +242,26 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
     }
   }
   const size_t base = arena_need(scheme, op, chunk, !dev);
-  // FrodoKEM on the tensor cores: operand tiles for A generated ahead, as far as the
-  // budget leaves room; none at all is a valid answer, and the one when the device has no memory for
-  // them.  A profiled batch above the size that is generated whole takes none, so that its stages are timed apart.
-  // Nor does a batch beside an open service: a front block (512 threads, 89-128 registers, 120 KB) does not fit
-  // on an SM that holds a CTA of the service (256 x 128 registers, 107 KB) and would wait until the
-  // service's launch ends; the kernels of the path without tiles fit beside one.
+  // FrodoKEM on the tensor cores: operand tiles for A generated ahead, as far as the budget leaves room and
+  // the arena holds them or can be grown (not against the device's refusal, during a capture, or after
+  // dpkem_ctx_reserve); none at all is a valid answer.  A profiled batch above the size that is generated
+  // whole takes none, so that its stages are timed apart.  Nor does a batch beside an open service: a
+  // front block (512 threads, 89-128 registers, 120 KB) does not fit on an SM that holds a CTA of the service
+  // (256 x 128 registers, 107 KB) and would wait until the service's launch ends; the kernels of the
+  // path without tiles fit beside one.
   const bool frodo_tc = scheme <= DPKEM_FRODO976AES && form == DPKEM_FORM_TC && open_services(c->device).load() == 0;
   size_t tile_cap = 0;
-  if (frodo_tc && c->budget / npipe > base + kAlign) {
-    const size_t room = (c->budget - (base + kAlign) * npipe) / npipe / frodo_ahead_bytes();
-    tile_cap = (size_t)frodo_ahead_count((int)chunk, room);
-    if (c->profile && tile_cap < chunk) tile_cap = 0;
+  if (frodo_tc) {
+    const size_t each = frodo_ahead_bytes();
+    auto room = [&](size_t bytes) { return bytes / npipe > base ? (bytes / npipe - base) / each : 0; };
+    size_t wish = (size_t)frodo_ahead_count((int)chunk, room(c->budget));
+    if (c->profile && wish < chunk) wish = 0;
+    CtxMem mem(c);
+    if (wish && !capturing(st)) c->arena.want(up(base + wish * each) * npipe, c->budget, mem);
+    tile_cap = std::min(wish, (size_t)frodo_ahead_count((int)chunk, room(c->arena.bytes)));
   }
-  size_t per_pipe = up(base + tile_cap * frodo_ahead_bytes());
-  int rc = ensure_arena(c, per_pipe * npipe);
-  if (rc == DPKEM_ENOMEM && tile_cap) {
-    tile_cap = 0;
-    per_pipe = up(base);
-    rc = ensure_arena(c, per_pipe * npipe);
-  }
+  const size_t per_pipe = up(base + tile_cap * frodo_ahead_bytes());
+  const int rc = ensure_arena(c, per_pipe * npipe, st);
   if (rc) return rc;
   cudaError_t e = cudaStreamWaitEvent(st, c->last, 0);
   if (e != cudaSuccess) return cuda_status(e);
@@ -272,7 +287,7 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
     if (edge && (k == 0 || k + 1 == (size_t)npipe)) m = std::min(edge, n - first);
     const int j = (int)(k % (size_t)npipe);
     cudaStream_t sj = streams[j];
-    Carver cv{c->arena + (size_t)j * per_pipe};
+    Carver cv{c->arena.base + (size_t)j * per_pipe};
     const uint8_t *d_in0, *d_in1 = nullptr;
     uint8_t *d_out0, *d_out1 = nullptr;
     FrodoBatch fb{};
@@ -316,7 +331,7 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
       fb.aes = scheme == DPKEM_FRODO976AES;
       fb.err = c->d_err;
       if (tile_cap) {
-        fb.atile = c->arena + (size_t)j * per_pipe + base;
+        fb.atile = c->arena.base + (size_t)j * per_pipe + base;
         fb.ahead = frodo_ahead_count((int)m, tile_cap);
         fb.queue = c->d_err + (1 + j) * kQueueStride;
       }
@@ -405,11 +420,11 @@ int run_shared(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8
   // With A in memory, the tensor-core form runs the products as one GEMM on tiled operands.
   const bool gemm = amat && form == DPKEM_FORM_TC;
   const size_t tiles = gemm ? up(frodo_gemm_ab_bytes()) + up(frodo_gemm_s_bytes(chunk)) : 0;
-  int rc = ensure_arena(c, arena_need(scheme, op, chunk, false) + kAlign + tiles);
+  int rc = ensure_arena(c, arena_need(scheme, op, chunk, false) + kAlign + tiles, st);
   if (rc) return rc;
   cudaError_t e = cudaStreamWaitEvent(st, c->last, 0);
   if (e != cudaSuccess) return cuda_status(e);
-  Carver cv{c->arena};
+  Carver cv{c->arena.base};
   FrodoBatch fb{};
   fb.rw = cv.take<uint16_t>(chunk * frodo::RW * 2);
   fb.kk = cv.take<uint8_t>(chunk * 24);
@@ -521,7 +536,9 @@ int dpkem_ctx_reserve(dpkem_ctx *c, size_t bytes) {
   if (!c) return set_status(DPKEM_EINVAL);
   std::lock_guard<std::mutex> lock(c->mu);
   if (cudaSetDevice(c->device) != cudaSuccess) return set_status(cuda_status(cudaErrorInvalidDevice));
-  return set_status(ensure_arena(c, bytes));
+  const int rc = ensure_arena(c, bytes);
+  if (rc == DPKEM_OK) c->arena.fix();
+  return set_status(rc);
 }
 
 size_t dpkem_mixed_bytes(int scheme, size_t n) {
@@ -539,7 +556,7 @@ int dpkem_selftest_timeout(dpkem_ctx *c, int which) {
   if (rc) return set_status(rc);
   cudaStream_t st = c->stream;
   cudaError_t e = cudaStreamWaitEvent(st, c->last, 0);
-  if (e == cudaSuccess) e = mixed::selftest_timeout(which, c->arena, c->arena_bytes, c->d_err, st);
+  if (e == cudaSuccess) e = mixed::selftest_timeout(which, c->arena.base, c->arena.bytes, c->d_err, st);
   if (e == cudaSuccess) e = cudaEventRecord(c->last, st);
   uint32_t err = 0;
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -563,8 +580,9 @@ int dpkem_ctx_destroy(dpkem_ctx *c) {
   if (!c) return set_status(DPKEM_EINVAL);
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->last) cudaEventSynchronize(c->last);
-  if (c->arena) cudaFree(c->arena);
+  CtxMem mem(c);
+  if (c->last) mem.drain();
+  c->arena.free_all(mem);
   if (c->d_err) cudaFree(c->d_err);
   if (c->last) cudaEventDestroy(c->last);
   for (int j = 0; j < kPipeChunks; j++) {
@@ -658,7 +676,7 @@ static int mixed_batch(dpkem_ctx *c, int form, size_t n, const dpkem_request *re
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
   const mixed::Req *mr = reinterpret_cast<const mixed::Req *>(reqs);
   const size_t need = mixed::plan_bytes(mr, n, nullptr);
-  if ((rc = ensure_arena(c, need)) != DPKEM_OK) return set_status(rc);
+  if ((rc = ensure_arena(c, need, st)) != DPKEM_OK) return set_status(rc);
   cudaError_t e = cudaStreamWaitEvent(st, c->last, 0);
   int grid = 0;
   if (e == cudaSuccess) e = persistent_grid(c, &grid);
@@ -666,7 +684,7 @@ static int mixed_batch(dpkem_ctx *c, int form, size_t n, const dpkem_request *re
   const size_t tb = mixed::plan_table_bytes(mr, n);
   uint8_t *stage = e == cudaSuccess ? stage_for(c, 0, tb) : nullptr;
   if (e == cudaSuccess)
-    e = mixed::plan_build(mr, n, form, grid, c->arena, c->arena_bytes, c->d_err, st, plan.data(), key, first, stage,
+    e = mixed::plan_build(mr, n, form, grid, c->arena.base, c->arena.bytes, c->d_err, st, plan.data(), key, first, stage,
                           stage ? c->h_stage_bytes[0] : 0);
   if (e == cudaSuccess && stage) stage_used(c, 0, st);
   if (e == cudaSuccess) e = mixed::plan_launch(plan.data(), n, grid, st);
@@ -776,9 +794,9 @@ int dpkem_coins(dpkem_ctx *c, size_t n, size_t len, uint64_t first, const char *
     const size_t m = std::min(chunk, n - f);
     b.n = (int)m;
     b.first = first + f;
-    b.out = c->arena;
+    b.out = c->arena.base;
     if ((e = coins_generate(b, st)) != cudaSuccess) return set_status(cuda_status(e));
-    if ((e = cudaMemcpyAsync(out + f * len, c->arena, m * len, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+    if ((e = cudaMemcpyAsync(out + f * len, c->arena.base, m * len, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return set_status(cuda_status(e));
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return set_status(cuda_status(e));
   }

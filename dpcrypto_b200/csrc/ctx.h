@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "../../include/dpkem.h"
+#include "arena.h"
 #include "common.cuh"
 
 struct dpkem_ctx {
@@ -21,8 +22,7 @@ struct dpkem_ctx {
   cudaEvent_t pev[16] = {};
   cudaStream_t aux[16] = {};    // a second stream per pipeline slot and its fork / join events
   cudaEvent_t fork_ev[16] = {}, join_ev[16] = {};
-  uint8_t *arena = nullptr;
-  size_t arena_bytes = 0;
+  dpkem::Arena arena;
   uint32_t *d_err = nullptr;
   int max_ctas = 0;  // persistent launches use at most this many CTAs (0: two per SM)
   uint8_t *h_stage[16] = {};      // pinned plan-table images, one per pipeline slot
@@ -48,7 +48,9 @@ struct Sizes {
 
 int set_status(int s);                      // records the calling thread's last status
 bool scheme_sizes(int scheme, Sizes *z);    // object sizes of a scheme; false if unknown
-int ensure_arena(dpkem_ctx *c, size_t bytes);  // grows the context's device arena
+// Grows the context's device arena.  st, if given, is the stream that the arena's memory is used on: one that
+// is being captured gets no growth, and what it records stays allocated.
+int ensure_arena(dpkem_ctx *c, size_t bytes, cudaStream_t st = nullptr);
 int cuda_status(cudaError_t e);             // DPKEM_OK or DPKEM_ECUDA (clears the error)
 // Services open on a device (serve.cu): their launches hold CTAs for as long as requests come.
 std::atomic<int> &open_services(int device);

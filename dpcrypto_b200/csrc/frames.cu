@@ -209,7 +209,7 @@ int frames_submit(dpkem_ctx *c, int form, const uint8_t *req, size_t req_bytes, 
   for (size_t k = 0; k < gs.size() && e == cudaSuccess; k++) {
     const Group &g = gs[k];
     cudaStream_t sj = c->pipe[k % npipe];
-    uint8_t *d_req = c->arena + (k % npipe) * region;
+    uint8_t *d_req = c->arena.base + (k % npipe) * region;
     uint8_t *d_resp = d_req + up(g.req_len);
     uint8_t *d_plan = d_resp + up(g.resp_len);
     const std::vector<mixed::Req> rq = group_reqs(fr, g, d_req, d_resp);

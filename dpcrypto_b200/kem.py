@@ -342,7 +342,8 @@ class Engine:
         return ss
 
     def reserve(self, nbytes: int):
-        """Grow this engine's device arena to nbytes now, outside any latency-critical call."""
+        """Grow this engine's device arena to nbytes now, outside any latency-critical call.  FrodoKEM's
+        operand tiles then take what is left of it and never grow it (include/dpkem.h)."""
         self._check(self._lib.dpkem_ctx_reserve(self._h, nbytes), "reserve")
 
     def set_max_ctas(self, max_ctas: int):

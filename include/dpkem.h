@@ -59,7 +59,12 @@ enum { DPKEM_FORM_DP4A = 0, DPKEM_FORM_INT32 = 1, DPKEM_FORM_TC = 2 };
 typedef struct dpkem_ctx dpkem_ctx;
 
 /* Create a context on `device` whose scratch arena may use at most `hbm_budget_bytes`
- * (0 = default 8 GiB).  Batches larger than the budget allows run in chunks. */
+ * (0 = default 8 GiB).  Batches larger than the budget allows run in chunks.  FrodoKEM batches with a key per
+ * instance in the tensor-core form also keep operand tiles there, 2,162,688 bytes an instance for all of up to
+ * 1,024 instances and for 296 to 591 of a larger batch (of each chunk, for host buffers): 2.2 GB for a batch
+ * of 1,024, 1.4 GB for 8,192, up to 6.5 GB for host batches of 2,048 and more.  Tiles are optional: with a smaller
+ * budget, or where the device refuses the memory (it is asked once for a size), the batch runs
+ * with fewer or none, and slower. */
 int dpkem_ctx_create(dpkem_ctx **out, int device, size_t hbm_budget_bytes);
 int dpkem_ctx_destroy(dpkem_ctx *ctx);
 /* Cap the CTAs of this context's persistent launches (mixed batches, graphs, frames):
@@ -69,7 +74,10 @@ int dpkem_ctx_set_max_ctas(dpkem_ctx *ctx, int max_ctas);
 
 /* Grow the context's device arena to at least `bytes` now (within its HBM budget), so
  * that no later call has to: regrowing frees the old arena, which waits for the whole
- * device.  dpkem_mixed_bytes(scheme, n) is the arena a mixed batch of n requests of that
+ * device.  From then on operand tiles (dpkem_ctx_create) take what a call's scratch (about 32 KB an instance
+ * for FrodoKEM) leaves of the arena and never grow it.  A stream capture never grows it either: calls to be
+ * captured need a reserved arena, and memory that a capture has recorded stays allocated until the
+ * context is destroyed.  dpkem_mixed_bytes(scheme, n) is the arena a mixed batch of n requests of that
  * scheme needs (Frodo requests need the most); 0 for an unknown scheme. */
 int dpkem_ctx_reserve(dpkem_ctx *ctx, size_t bytes);
 
