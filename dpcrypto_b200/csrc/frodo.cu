@@ -427,11 +427,17 @@ size_t frodo_ahead_bytes() { return ahead::A_BYTES; }
 // others; an ahead part of 296 .. 591 instances fills the SMs that the prologue leaves free, and
 // leaves whole waves.  Measured ms, encaps: n = 768 all ahead 2.80, 176 ahead 3.45; 1,024 all
 // 3.65, 432 ahead 3.83, none 4.6; 8,192: none 26.99, 200 ahead 26.23, 350 25.83, 496 25.65, 560 25.87.
+// With scratch for fewer, as many as leave whole waves to the A stage, or none: other numbers cost more than they
+// save, and so does a part of a batch of 1,025 .. kFrontTenMax, whose chains then hold the SMs.  ms, none / that
+// many / another number, encaps: n = 64 1.42 / - / 16 1.49; 768 3.61 / 176 3.03, 472 2.94 / 4 3.68, 296 3.38;
+// 1,024 4.14 / 136 4.01, 432 3.72 / 64 4.20; 4,096 13.7 / 248 14.4 / 128 14.6; 8,192 27.0 / 200 26.2.
 constexpr int kAheadAll = 1024;
 
 int frodo_ahead_count(int n, size_t cap) {
-  const int wave = 2 * device_sms(), m = n <= kAheadAll ? n : wave + n % wave;
-  return (int)std::min<size_t>(m, cap);
+  const int wave = 2 * device_sms(), rest = n % wave, most = n <= kAheadAll ? n : wave + rest;
+  if (cap >= (size_t)most) return most;
+  if ((int)cap < rest || (n > kAheadAll && n <= kFrontTenMax)) return 0;
+  return rest + ((int)cap - rest) / wave * wave;
 }
 
 cudaError_t frodo_keypair(const FrodoBatch &b, int form, cudaStream_t st) {
