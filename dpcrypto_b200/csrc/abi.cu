@@ -869,7 +869,7 @@ int dpkem_frodo_dec_shared(dpkem_ctx *c, int scheme, int form, size_t n, const u
 }
 
 int dpkem_keccak_f1600_lanes(dpkem_ctx *c, int lanes, size_t n, const uint64_t *in, uint64_t *out, int perms) {
-  if (!c || (lanes != 1 && lanes != 2 && lanes != 5 && lanes != 25) || perms < 0 || n > (size_t)INT32_MAX)
+  if (!c || (lanes != 1 && lanes != 2 && lanes != 5 && lanes != 10 && lanes != 25) || perms < 0 || n > (size_t)INT32_MAX)
     return set_status(DPKEM_EINVAL);
   if (n == 0) return set_status(DPKEM_OK);
   if (!in || !out || (reinterpret_cast<uintptr_t>(in) & 7) || (reinterpret_cast<uintptr_t>(out) & 7))
@@ -882,7 +882,7 @@ int dpkem_keccak_f1600_lanes(dpkem_ctx *c, int lanes, size_t n, const uint64_t *
 }
 
 int dpkem_probe_keccak_chain(dpkem_ctx *c, int lanes, int states, int perms, double *ms) {
-  if (!c || !ms || (lanes != 1 && lanes != 2 && lanes != 5 && lanes != 25) || states <= 0 || perms <= 0)
+  if (!c || !ms || (lanes != 1 && lanes != 2 && lanes != 5 && lanes != 10 && lanes != 25) || states <= 0 || perms <= 0)
     return set_status(DPKEM_EINVAL);
   std::lock_guard<std::mutex> lock(c->mu);
   cudaSetDevice(c->device);

@@ -411,7 +411,7 @@ class Engine:
 
     def keccak_lanes(self, lanes: int, states, perms: int = 1):
         """`perms` Keccak-f[1600] permutations of each row of `states` (an n x 25 torch CUDA
-        tensor of 64-bit lanes) in the given lanes-per-state layout (1, 2, 5 or 25); returns a new
+        tensor of 64-bit lanes) in the given lanes-per-state layout (1, 2, 5, 10 or 25); returns a new
         tensor.  The calling torch stream's pending work is synchronised first."""
         import torch
 

@@ -235,7 +235,8 @@ int dpkem_frodo_dec_shared(dpkem_ctx *ctx, int scheme, int form, size_t n, const
                            const uint16_t *amat, uint8_t *ss, void *stream);
 
 /* Keccak-f[1600] in each lanes-per-state layout the sponge stages use (1: a thread per state,
- * 2: a bit-interleaved lane pair, 5: five lanes of a warp, 25: a warp per state): `perms` permutations
+ * 2: a bit-interleaved lane pair, 10: ten lanes of a warp, 25: a warp per state; and 5: five lanes, which no
+ * stage uses): `perms` permutations
  * applied to each of n states (25 little-endian 64-bit lanes each, device pointers, 8-byte
  * aligned); returns when done.  No counterpart in the reference (its permutation is
  * KeccakF1600_StatePermute, FrodoKEM976-GPU/src/shake.cu:66-331, one thread per state). */
