@@ -20,9 +20,9 @@
 // conflict.  Hence the buffer's shape: slot s of all six (state, half) pairs c is one line of
 // 208 bytes, rows 0..3 at 16 c, row 4 at 96 + 4 c.  The stores of a slot then hit 30 different banks,
 // and the 208-byte stride (13 x 16) puts the eight 16-byte loads of every quarter warp on
-// different banks too.  Measured, us per permutation of a dependent chain (a warp per state / five
-// lanes / pair / here): 6 states 2.09 / 3.38 / 2.53 / 2.04, 1,024 2.42 / 3.38 / 2.55 / 2.11, 2,048
-// 4.20 / 3.56 / 2.55 / 2.35, 4,096 6.76 / 4.50 / 2.58 / 2.97, 8,192 13.5 / 6.81 / 2.66 / 5.35.
+// different banks too.  Measured, us per permutation of a dependent chain (dpkem_probe_keccak_chain; a warp per
+// state / five lanes / pair / here): 6 states 2.02 / 3.07 / 2.50 / 1.91, 1,024 2.27 / 3.08 / 2.51 / 1.95, 2,048
+// 4.11 / 3.26 / 2.51 / 2.01, 4,096 6.69 / 3.92 / 2.53 / 2.54, 8,192 13.4 / 6.28 / 2.62 / 4.87.
 //
 // Lanes 30 and 31 repeat lanes 0 and 1 (the same loads, stores of the same words); callers drop their
 // writes to global memory.  Every lane of the warp must execute every call.
@@ -108,8 +108,8 @@ __device__ __forceinline__ void round10(uint32_t (&a)[5], const Lanes &k, uint32
   // lane's loads above have returned (the shuffled values depend on them).
 }
 
-// U rounds per iteration (us per permutation, 512 / 4,096 states: 1 round 2.33 / 3.13, 2 2.20 / 3.09,
-// 4 2.11 / 3.02, 8 2.11 / 2.97, 24 2.02 / 2.71).  Eight where a stage inlines several permutations (24
+// U rounds per iteration (us per permutation of a chain, 512 / 4,096 states: 1 round 2.26 / 3.05, 2 2.07 / 3.03,
+// 4 2.06 / 2.93, 8 2.02 / 2.91, 24 1.92 / 2.55).  Eight where a stage inlines several permutations (24
 // rounds of each would not stay in the instruction cache), 24 where it has one.
 template <int U = 8>
 __device__ __forceinline__ void f1600(uint32_t (&a)[5], const Lanes &k) {

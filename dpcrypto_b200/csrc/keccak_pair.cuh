@@ -7,7 +7,7 @@
 // round is 90 integer operations and 17 shuffles per thread instead of 180 operations on
 // one thread.  Where a stage has one warp per SM sub-partition, a warp is bound by its own
 // issue rate (the 16-lane integer pipe takes a warp instruction every two cycles), so
-// halving the instructions per state shortens a sponge chain: 2.55 us a permutation against 4.6
+// halving the instructions per state shortens a sponge chain: 2.51 us a permutation against 4.55
 // on one thread, at the same 135 integer operations a state.
 //
 // Sponge bytes (msponge.cuh's Multi<2>) cross the boundary through to_slice / half_to_slice (a
@@ -78,10 +78,11 @@ __device__ __forceinline__ void round(uint32_t (&a)[25], uint32_t rc, uint32_t q
   a[0] ^= rc;
 }
 
-// Eight rounds per iteration: one warp per sub-partition waits for its own shuffles, and a longer
+// Four rounds per iteration: one warp per sub-partition waits for its own shuffles, and a longer
 // body lets a round's first operations start among the previous round's last.  Measured us per
-// permutation of a chain (512 states; 8,192): 1 round 3.09 (3.18), 2 2.75 (2.93), 4 2.59 (2.79), 8
-// 2.55 (2.66), 24 3.64 (4.24: past the instruction cache).
+// permutation of a chain (512 states; 8,192): 1 round 2.99 (3.05), 2 2.67 (2.83), 4 2.51 (2.62), 8
+// 2.47 (2.56; not measured in the stages, which inline several permutations), 24 4.01 (4.13: past the
+// instruction cache).
 __device__ __forceinline__ void f1600(uint32_t (&a)[25], int p) {
   const uint32_t q = 1u - (uint32_t)p;
 #pragma unroll 4
