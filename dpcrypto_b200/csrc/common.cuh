@@ -36,13 +36,12 @@ __host__ __device__ constexpr Params params(int level) {
 }  // namespace saber
 
 inline int device_sms() {
-  static int sms = 0;
-  if (!sms) {
+  static const int sms = [] {
     int dev = 0, m = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
-    sms = m > 0 ? m : 1;
-  }
+    return m > 0 ? m : 1;
+  }();
   return sms;
 }
 // For kernels whose warps have unlike roles.  A block's warp w runs on SM sub-partition (its first warp

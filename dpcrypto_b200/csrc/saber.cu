@@ -2,6 +2,7 @@
 // launch per stage over n instances.  The stage bodies live in saber_dev.cuh (shared with
 // the persistent mixed-batch kernel); these wrappers only map blockIdx/threadIdx to instances.
 #include <algorithm>
+#include <atomic>
 
 #include "saber_chain.cuh"
 #include "saber_dev.cuh"
@@ -323,12 +324,15 @@ cudaError_t launch_product(const SaberBatch &b, int form, cudaStream_t st, bool 
       // another, so a grid larger than what is resident only queues; TMEM (32 columns per
       // CTA) fits 16 CTAs per SM.
       if ((e = prep(product_tc_persistent_kernel<L, MODE>, bytes)) != cudaSuccess) return e;
-      static bool carved = false;  // per process and instantiation
-      if (!carved) {
+      static std::atomic<uint64_t> carved{0};  // per instantiation, a bit per device
+      int dev = 0;
+      if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+      const uint64_t bit = 1ull << (dev & 63);
+      if (!(carved.load(std::memory_order_relaxed) & bit)) {
         if ((e = cudaFuncSetAttribute(product_tc_persistent_kernel<L, MODE>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess)
           return e;
-        carved = true;
+        carved.fetch_or(bit, std::memory_order_relaxed);
       }
       const int grid = std::min(b.n, device_sms() * std::min(per_sm, kProductCtas<L>));
       return launch_next(follows, product_tc_persistent_kernel<L, MODE>, grid, 256, bytes, st, b);
