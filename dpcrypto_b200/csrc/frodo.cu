@@ -348,15 +348,11 @@ cudaError_t launch_front(const FrodoBatch &b, bool halve, cudaStream_t st) {
   return launch_front_ns<STAGE, 0, false>(b, st);
 }
 
-// Column blocks per product CTA: the whole chip has to be busy with few instances; with many,
-// a CTA per instance part of four blocks reads S' three times instead of twelve.
 template <int MODE>
 cudaError_t launch_product(const FrodoBatch &b, cudaStream_t st) {
   cudaError_t e;
-  const int nb = b.ahead * 12 <= 592 ? 1 : b.ahead * 6 <= 592 ? 2 : 4;
-  const uint32_t cols = nb <= 2 ? 32 : 64;
   if ((e = set_smem(ahead::product_kernel<MODE>, ahead::PLayout::total)) != cudaSuccess) return e;
-  ahead::product_kernel<MODE><<<b.ahead * (ahead::BLKS / nb), 256, ahead::PLayout::total, st>>>(b, nb, cols);
+  ahead::product_kernel<MODE><<<b.ahead * (ahead::BLKS / ahead::P_NB), 256, ahead::PLayout::total, st>>>(b);
   return cudaGetLastError();
 }
 template <bool RAW>

@@ -4,7 +4,7 @@
 // instance) need not wait for the prologue (up to 348 dependent ones, one to a few warps'
 // worth of issue slots).  The front kernel runs both: a few blocks the sponge chains, all others
 // the rows of A, stored as operand tiles.  The product of an instance is then a pass of
-// tcgen05 MMAs over its 2.1 MB of tiles, split over as many CTAs as the batch leaves room for.
+// tcgen05 MMAs over its 2.1 MB of tiles, on three CTAs.
 //
 //   front    blocks [0, chain): the prologue's sponges; [chain, chain + absorb): decaps'
 //            ciphertext pre-absorb; the rest: 256 rows of A each, a row per thread
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(32) kp_seed_kernel(FrodoBatch b) {
 }
 
 // ---------------------------------------------------------------- product S'A
-// CTA (256 threads) = one instance, column blocks [b0, b0 + nb).  Warp 0 lane 0 moves the tiles
+// CTA (256 threads) = one instance, P_NB column blocks from b0 on.  Warp 0 lane 0 moves the tiles
 // (one bulk copy each) through an NST-stage mbarrier ring, warp 1 lane 0 issues the MMAs (per
 // 32 rows: bytes 0..127 and 128..167 of the block, N = 8), the CTA of the last block also forms
 // V = S'B on warps 2..7 meanwhile.  All eight warps read the accumulators back.
@@ -270,6 +270,11 @@ __global__ void __launch_bounds__(32) kp_seed_kernel(FrodoBatch b) {
 // the errors.  PM_ENC: ciphertext.  PM_DEC: compare, an OR into the fail word.
 enum PMode : int { PM_RAW = 0, PM_ENC = 1, PM_DEC = 2 };
 constexpr int P_NST = 4;
+// Column blocks of a CTA: four read S' three times an instance; narrower CTAs for few instances gain nothing.  us, 1 / 2 / 4
+// blocks, encaps: n = 1 745 / 744 / 744, 32 783 / 781 / 778, 128 846 / 842 / 833, 1,024 3,786 / 3,722 / 3,700; decaps at
+// 1,024 3,618 / 3,536 / 3,503.
+constexpr int P_NB = 4;
+constexpr uint32_t P_TMEM = 64;
 
 struct PLayout {
   static constexpr int sp = 0;                                   // S' operand, 62 * 128
@@ -282,12 +287,13 @@ struct PLayout {
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b, int nb, uint32_t tmem_cols) {
+__global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b) {
   using L = PLayout;
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int op = MODE == PM_DEC ? OP_DEC : OP_ENC;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int parts = BLKS / nb, inst = blockIdx.x / parts, b0 = (blockIdx.x % parts) * nb, b1 = b0 + nb;
+  constexpr int parts = BLKS / P_NB, nst = P_NB * TILES;
+  const int inst = blockIdx.x / parts, b0 = (blockIdx.x % parts) * P_NB, b1 = b0 + P_NB;
   const Inst v = inst_of(b, inst, op);
   const uint8_t *tiles = b.atile + (size_t)inst * A_BYTES;
   uint8_t *sp = smem + L::sp;
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b, int nb, u
   uint32_t(*red)[64] = reinterpret_cast<uint32_t(*)[64]>(smem + L::red);
   const uint16_t *rw = v.rw;
   if (warp == 0) {
-    tmem_alloc(tslot, tmem_cols);
+    tmem_alloc(tslot, P_TMEM);
     tmem_relinquish();
   }
   if (tid == 32) {
@@ -319,7 +325,6 @@ __global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b, int nb, u
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *tslot;
-  const int nst = nb * TILES;
   bool ok = true;
   if (warp == 0) {
     if (lane == 0) {  // producer
@@ -429,7 +434,7 @@ __global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b, int nb, u
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tbase, tmem_cols);
+    tmem_dealloc(tbase, P_TMEM);
   }
 }
 
