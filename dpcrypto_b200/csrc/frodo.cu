@@ -335,10 +335,13 @@ cudaError_t launch_front_ns(const FrodoBatch &b, cudaStream_t st) {
   return b.aes ? launch_front_g<STAGE, NS, HALVE, fdev::AesRowsFull>(b, st)
                : launch_front_g<STAGE, NS, HALVE, fdev::ShakeRows>(b, st);
 }
-// Ten lanes per state up to kFrontTenMax: beyond, the chains' SMs on one lane cost less (a
-// permutation is 135 integer instructions per state there, 160 on ten lanes) than their shorter latency gains,
-// since the rows fill the other SMs meanwhile.  `halve` (encaps, keypair): stop the stream after S',
-// tail_kernel runs the rest.
+// Ten lanes per state up to kFrontTenMax; beyond, one: a permutation is 135 integer instructions per state there, 160 on
+// ten lanes, whose chain blocks hold more SM time, while the rows fill the other SMs as long as one lane's
+// chains last.  Between about 2,000 and 4,000 it depends on the rows ahead (n mod 296): few of them end before
+// one lane's chains do.  ms, ten lanes / one, encaps: 1,025 3.72 / 4.30, 2,072 (0 mod 296) 7.45 / 7.77, 2,600 8.82 / 8.74, 3,700
+// 12.44 / 12.26, 3,848 (0) 13.48 / 13.04, 4,096 13.64 / 13.13, 5,000 16.64 / 15.95; decaps: 1,025 3.46 / 4.08, 2,072 6.74 / 7.52,
+// 3,700 11.92 / 11.95, 3,848 12.34 / 12.74, 4,096 13.15 / 12.84; keypair: 1,536 5.31 / 5.57, 2,000 6.89 / 6.73, 2,072 7.14 / 7.40,
+// 4,096 13.75 / 13.39.  `halve` (encaps, keypair): stop the stream after S', tail_kernel runs the rest.
 constexpr int kFrontTenMax = 4096;
 template <int STAGE>
 cudaError_t launch_front(const FrodoBatch &b, bool halve, cudaStream_t st) {
@@ -363,8 +366,8 @@ cudaError_t launch_product_kp(const FrodoBatch &b, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Whether the batch runs the halved stream and the stepped tail: every instance's products must
-// come raw from product_kernel, and the sponges must be on a warp per state.
+// Whether the batch runs the halved stream and the stepped tail (ten lanes per state): every instance's
+// products must come raw from product_kernel.
 bool halved(const FrodoBatch &b) { return b.ahead == b.n; }
 bool use_ahead(const FrodoBatch &b, int form) { return form == FORM_TC && b.atile && b.ahead > 0 && !b.amat; }
 
