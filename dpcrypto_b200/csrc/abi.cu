@@ -914,7 +914,8 @@ int dpkem_set_tuning(const char *key, int value) {
   const bool zero_ok = k == "pipe_priority" || k == "saber_pair_max" || k == "saber_five_max" ||
                        k == "saber_finish_five_max" || k == "frodo_five_max" || k == "frodo_ss_five_max" ||
                        k == "saber_tc_ctas_per_sm" || k == "saber_warp_max" || k == "saber_finish_warp_max" ||
-                       k == "frodo_warp_max" || k == "frodo_ss_warp_max" || k == "mixed_warp_max";
+                       k == "frodo_warp_max" || k == "frodo_ss_warp_max" || k == "frodo_pair_max" ||
+                       k == "mixed_warp_max";
   if (value == 0 && !zero_ok) return set_status(DPKEM_EINVAL);
   if (k == "thread_block") {
     if (value % 32 || value > 256) return set_status(DPKEM_EINVAL);
@@ -947,6 +948,8 @@ int dpkem_set_tuning(const char *key, int value) {
     t.saber_finish_warp_max = value;
   } else if (k == "frodo_warp_max") {
     t.frodo_warp_max = value;
+  } else if (k == "frodo_pair_max") {
+    t.frodo_pair_max = value;
   } else if (k == "frodo_ss_warp_max") {
     t.frodo_ss_warp_max = value;
   } else if (k == "saber_tc_ctas_per_sm") {
@@ -972,7 +975,7 @@ int dpkem_get_tuning(const char *key, int *value) {
                {"saber_finish_warp_max", t.saber_finish_warp_max}, {"saber_five_max", t.saber_five_max},
                {"saber_finish_five_max", t.saber_finish_five_max}, {"frodo_warp_max", t.frodo_warp_max},
                {"frodo_ss_warp_max", t.frodo_ss_warp_max}, {"frodo_five_max", t.frodo_five_max},
-               {"frodo_ss_five_max", t.frodo_ss_five_max}, {"saber_tc_ctas_per_sm", t.saber_tc_ctas_per_sm}};
+               {"frodo_ss_five_max", t.frodo_ss_five_max}, {"frodo_pair_max", t.frodo_pair_max}, {"saber_tc_ctas_per_sm", t.saber_tc_ctas_per_sm}};
   for (const auto &kn : knobs)
     if (k == kn.name) {
       *value = kn.v;

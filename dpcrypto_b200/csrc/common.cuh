@@ -48,7 +48,7 @@ inline int device_sms() {
 // slot + w) mod 4, so with fixed roles the long ones of an SM's blocks pile up on the same
 // sub-partitions; this tells a block (all its threads) whether to exchange them: every other four slots.
 __device__ __forceinline__ bool exchange_roles() {
-  if (gridDim.x <= 128) return false;  // a block an SM
+  if (gridDim.x <= 128) return false;  // fewer blocks than SMs: none shares one
   __shared__ uint32_t slot;
   if (threadIdx.x == 0) asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
   __syncthreads();
@@ -84,6 +84,9 @@ struct Tuning {
   // largest Frodo batch whose H(pk) and final hash run on a warp per state / ten lanes (0: never)
   int frodo_ss_warp_max = 512;
   int frodo_ss_five_max = 3072;
+  // largest Frodo batch above those whose encaps / keypair prologue and hashes run on a lane pair (0: never): a
+  // warp of sixteen on each of 148 x 4 SM sub-partitions (final hashes at 8,192 0.39 ms against 0.55 on one lane)
+  int frodo_pair_max = 148 * 4 * 16;
   int saber_tc_ctas_per_sm = 6; // persistent Saber tensor-core product CTAs per SM (0: a CTA per instance)
 };
 Tuning &tuning();

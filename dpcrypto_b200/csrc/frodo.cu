@@ -135,22 +135,20 @@ __global__ void __launch_bounds__(256, 2) kp_as_tc_kernel(FrodoBatch b) {
 
 inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
-// Lanes per state of a hash stage: a warp per state up to warp_max (frodo_ss_warp_max), ten lanes
-// up to five_max (frodo_ss_five_max; the name is from a layout of five), a pair up to
-// kPairMax (a warp of pairs per SM sub-partition: final hashes at 8,192 0.39 ms against 0.55 on one
-// lane), else one (false: the caller launches that).
-constexpr int kPairMax = 148 * 4 * 16;
+// Lanes per state of a hash stage: a warp per state up to frodo_ss_warp_max, ten lanes up to frodo_ss_five_max (the
+// name is from a layout of five), a pair up to frodo_pair_max, else one (false: the caller launches that).
 template <int STAGE>
-bool launch_multi(const FrodoBatch &b, int warp_max, int five_max, cudaStream_t st) {
-  if (b.n <= warp_max) {
+bool launch_multi(const FrodoBatch &b, cudaStream_t st) {
+  const Tuning &t = tuning();
+  if (b.n <= t.frodo_ss_warp_max) {
     stage_multi_kernel<STAGE, 1><<<b.n, 32, 0, st>>>(b);
     return true;
   }
-  if (b.n <= five_max) {
+  if (b.n <= t.frodo_ss_five_max) {
     stage_multi_kernel<STAGE, 10><<<blocks_for(b.n, 3), 32, 0, st>>>(b);
     return true;
   }
-  if (b.n <= kPairMax) {
+  if (b.n <= t.frodo_pair_max) {
     stage_multi_kernel<STAGE, 2><<<blocks_for(b.n, 16), 32, 0, st>>>(b);
     return true;
   }
@@ -265,7 +263,7 @@ cudaError_t launch_kp_as(const FrodoBatch &b, int form, cudaStream_t st) {
 
 // The prologue without A's rows: on chain and helper warps up to frodo_warp_max / frodo_five_max (decaps,
 // whose ciphertext hash shares the SMs, at most to kDecChains), encaps and keypair on pairs up to
-// kPairMax; false above.  us of the whole call under one key, chains / pairs, encaps: n = 4,096 1,508 / 1,719,
+// frodo_pair_max; false above.  us of the whole call under one key, chains / pairs, encaps: n = 4,096 1,508 / 1,719,
 // 6,144 1,782 / 1,832, 7,000 1,903 / 1,853; chains / one lane, decaps: 1,024 655 / 1,544, 4,096 1,121 / 1,662, 4,871 (the
 // blocks that are resident at once end there) 1,327 / 1,696, 5,300 1,387 / 1,706, 5,700 1,609 / 1,721, 6,144
 // 1,816 / 1,738.
@@ -279,7 +277,7 @@ bool launch_prologue(const FrodoBatch &b, cudaStream_t st) {
     ahead::chains_kernel<ROLE><<<chain + absorb, 128, ahead::chain_smem(2), st>>>(b, chain);
     return true;
   }
-  if (ROLE == ahead::R_DEC || b.n > kPairMax) return false;
+  if (ROLE == ahead::R_DEC || b.n > tuning().frodo_pair_max) return false;
   stage_multi_kernel<ROLE == ahead::R_KEYPAIR ? 0 : 2, 2><<<blocks_for(b.n, 16), 32, 0, st>>>(b);
   return true;
 }
@@ -457,7 +455,7 @@ cudaError_t frodo_keypair(const FrodoBatch &b, int form, cudaStream_t st) {
     }
     mark(b, st);
     if (half) ahead::tail_kernel<OP_KEYPAIR><<<blocks_for(b.n, 3), 96, 0, st>>>(b);
-    else if (!launch_multi<1>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st))
+    else if (!launch_multi<1>(b, st))
       pk_hash_kernel<OP_KEYPAIR><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
     mark(b, st);
     return cudaGetLastError();
@@ -470,7 +468,7 @@ cudaError_t frodo_keypair(const FrodoBatch &b, int form, cudaStream_t st) {
                              : launch_kp_as<fdev::ShakeRows, fdev::KPT_NST>(b, form, st);
   if (e != cudaSuccess) return e;
   mark(b, st);
-  if (!launch_multi<1>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st)) pk_hash_kernel<OP_KEYPAIR><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
+  if (!launch_multi<1>(b, st)) pk_hash_kernel<OP_KEYPAIR><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
   mark(b, st);
   return cudaGetLastError();
 }
@@ -488,7 +486,7 @@ cudaError_t frodo_enc(const FrodoBatch &b, int form, cudaStream_t st) {
     if (b.ahead < b.n && (e = launch_sa<OP_ENC>(rest_of(b, b.ahead, OP_ENC), form, st)) != cudaSuccess) return e;
     mark(b, st);
     if (half) ahead::tail_kernel<OP_ENC><<<blocks_for(b.n, 3), 96, 0, st>>>(b);
-    else if (!launch_multi<3>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st))
+    else if (!launch_multi<3>(b, st))
       ss_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
     mark(b, st);
     return cudaGetLastError();
@@ -499,7 +497,7 @@ cudaError_t frodo_enc(const FrodoBatch &b, int form, cudaStream_t st) {
   cudaError_t e = launch_sa<OP_ENC>(b, form, st);
   if (e != cudaSuccess) return e;
   mark(b, st);
-  if (!launch_multi<3>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st)) ss_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
+  if (!launch_multi<3>(b, st)) ss_kernel<OP_ENC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
   mark(b, st);
   return cudaGetLastError();
 }
@@ -517,7 +515,7 @@ cudaError_t frodo_dec(const FrodoBatch &b, int form, cudaStream_t st) {
     if ((e = launch_product<ahead::PM_DEC>(b, st)) != cudaSuccess) return e;
     if (b.ahead < b.n && (e = launch_sa<OP_DEC>(rest_of(b, b.ahead, OP_DEC), form, st)) != cudaSuccess) return e;
     mark(b, st);
-    if (!launch_multi<4>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st))
+    if (!launch_multi<4>(b, st))
       ss_kernel<OP_DEC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
     mark(b, st);
     return cudaGetLastError();
@@ -527,7 +525,7 @@ cudaError_t frodo_dec(const FrodoBatch &b, int form, cudaStream_t st) {
   cudaError_t e = launch_sa<OP_DEC>(b, form, st);
   if (e != cudaSuccess) return e;
   mark(b, st);
-  if (!launch_multi<4>(b, tuning().frodo_ss_warp_max, tuning().frodo_ss_five_max, st)) ss_kernel<OP_DEC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
+  if (!launch_multi<4>(b, st)) ss_kernel<OP_DEC><<<blocks_for(b.n, tb), tb, 0, st>>>(b);
   mark(b, st);
   return cudaGetLastError();
 }

@@ -74,9 +74,8 @@ __global__ void __launch_bounds__(64) prologue_kernel(SaberBatch b, int first) {
   if (i < b.n) sdev::prologue_inst<L, OP>(inst_of<L>(b, i, OP), first + w);
 }
 
-// Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 10: ten lanes, three
-// instances per warp; NS = 2: a pair, sixteen).  The bit-interleaved ones leave the XOF bytes in
-// their form (b.sliced): converted there, a pair's 21 words a permutation made the l = 3 prologue of
+// Several lanes per state (msponge.cuh; NS = 1: a warp per instance; NS = 2: a pair, sixteen
+// instances per warp).  Pairs leave the XOF bytes in their form (b.sliced): converted there, a pair's 21 words a permutation made the l = 3 prologue of
 // 4,096 85 us against 77, and ten lanes' FireSaber prologue of 1,501 120 against 107; in the product's
 // staging they are two words a thread (2 us).
 template <int L, int OP, int NS>
@@ -182,7 +181,7 @@ cudaError_t launch_prologue(const SaberBatch &b, cudaStream_t st, bool follows, 
   }
 }
 
-// Encaps / keypair finish on several lanes per state, one warp per block.
+// Encaps / keypair finish on a warp (NS = 1) or a pair (2) per state, one warp per block.
 template <int L, int OP, int NS>
 __global__ void __launch_bounds__(32) finish_multi_kernel(SaberBatch b) {
   next_may_start();

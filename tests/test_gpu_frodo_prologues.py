@@ -67,3 +67,38 @@ def test_small_chain_limit(engine, oracle, form, n):
         idx = [0, 1, n - 1]
         h = lambda t: np.ascontiguousarray(t[idx].cpu().numpy())  # noqa: E731
         assert (h(got) == oracle.dec(0, h(bad), np.repeat(sk.cpu().numpy()[None], 3, 0), threads=THREADS)).all()
+
+
+BIG = 1 << 30
+PROLOGUES = {"chains": dict(frodo_warp_max=0, frodo_five_max=BIG),
+             "pair": dict(frodo_warp_max=0, frodo_five_max=0, frodo_pair_max=BIG),
+             "one": dict(frodo_warp_max=0, frodo_five_max=0, frodo_pair_max=0)}
+HASHES = {"warp": dict(frodo_ss_warp_max=BIG), "ten": dict(frodo_ss_warp_max=0, frodo_ss_five_max=BIG),
+          "pair": dict(frodo_ss_warp_max=0, frodo_ss_five_max=0, frodo_pair_max=BIG),
+          "one": dict(frodo_ss_warp_max=0, frodo_ss_five_max=0, frodo_pair_max=0)}
+
+
+# n = 50 and 67 leave partial groups of three, sixteen and thirty-two; the pair limit is common to both stages
+@pytest.mark.parametrize("n", [1, 50, 67])
+@pytest.mark.parametrize("scheme,form", [(d.FRODO976, d.FORM_DP4A), (d.FRODO976AES, d.FORM_INT32)])
+@pytest.mark.parametrize("prologue,hash_", [("chains", "warp"), ("chains", "ten"), ("chains", "pair"), ("chains", "one"),
+                                            ("pair", "pair"), ("pair", "warp"), ("one", "one"), ("one", "ten")])
+def test_layouts(engine, oracle, scheme, form, prologue, hash_, n):
+    kc = torch.empty((n, 64), dtype=torch.uint8, device="cuda")
+    ec = torch.empty((n, 24), dtype=torch.uint8, device="cuda")
+    engine.coins(n, 64, "prol-kp", first=n, out=kc)
+    engine.coins(n, 24, "prol-enc", first=n, out=ec)
+    h = lambda t: t.cpu().numpy()  # noqa: E731
+    pk_o, sk_o = oracle.keypair(scheme, h(kc), threads=THREADS)
+    ct_o, ss_o = oracle.enc(scheme, pk_o, h(ec), threads=THREADS)
+    bad = torch.from_numpy(ct_o).cuda()
+    bad[::2, 15743] ^= 128
+    rej_o = oracle.dec(scheme, h(bad), sk_o, threads=THREADS)
+    with d.kem.knobs(**{**HASHES[hash_], **PROLOGUES[prologue]}):
+        pk, sk = engine.keypair(scheme, kc, form)
+        ct, ss = engine.enc(scheme, pk, ec, form)
+        rej = engine.dec(scheme, bad, sk, form)
+        tc = engine.dec(scheme, bad, sk, d.FORM_TC)  # its final hash
+    assert (h(pk) == pk_o).all() and (h(sk) == sk_o).all()
+    assert (h(ct) == ct_o).all() and (h(ss) == ss_o).all()
+    assert (h(rej) == rej_o).all() and (h(tc) == rej_o).all()
