@@ -544,8 +544,12 @@ int dpkem_ctx_reserve(dpkem_ctx *c, size_t bytes) {
 size_t dpkem_mixed_bytes(int scheme, size_t n) {
   Sizes z;
   if (!scheme_sizes(scheme, &z) || n == 0) return 0;
-  std::vector<mixed::Req> rq(n, mixed::Req{scheme, OP_ENC, nullptr, nullptr, nullptr, nullptr});
-  return mixed::plan_bytes(rq.data(), n, nullptr);
+  size_t most = 0;  // the operations differ in their stages and in the size of a task
+  for (int op = OP_KEYPAIR; op <= OP_DEC; op++) {
+    const std::vector<mixed::Req> rq(n, mixed::Req{scheme, op, nullptr, nullptr, nullptr, nullptr});
+    most = std::max(most, mixed::plan_bytes(rq.data(), n, nullptr));
+  }
+  return most + 1024;  // a batch of all three rounds the tasks of each group up: at most eleven more
 }
 
 int dpkem_selftest_timeout(dpkem_ctx *c, int which) {
