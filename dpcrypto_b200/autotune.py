@@ -12,10 +12,12 @@ Knobs:
   pipe_priority      chunk streams with descending priorities (earlier chunks finish first)
   lanes per state    per sponge stage (Saber prologue, Saber encaps finish, Frodo prologue,
                      Frodo shared-secret hash) and batch size: a warp per state
-                     (*_warp_max), ten lanes (*_five_max), a lane pair (saber_pair_max,
-                     Saber only) or one lane.  Each layout is forced in turn at 64-16k
-                     instances (Frodo 64-8k) and timed with the stage timer; a layout covers batches up
-                     to the largest swept size at which it was the fastest
+                     (*_warp_max; not the Frodo prologue), ten lanes (*_five_max; the Frodo prologue on
+                     chain and helper warps), a lane pair (saber_pair_max; Frodo's, frodo_pair_max, is
+                     timed but not chosen: a warp of pairs per SM sub-partition) or one lane.
+                     Each layout is forced in turn at 64-16k instances (Frodo 64-8k, in the dot-product
+                     form, whose stages are those kernels at every size) and timed with the stage
+                     timer; a layout covers batches up to the largest swept size at which it was the fastest
   saber_tc_ctas_per_sm  persistent Saber tensor-core product (CTAs per SM) or a CTA per
                      instance (0)
   mixed_warp_max     groups of up to this many instances run their sponge stages as warp
@@ -155,10 +157,10 @@ def _child(u: int) -> dict:
     B = 4096
     res["frodo_b4096_ms"] = frodo_time(B)[1]
     sweep = {}
-    # the thread-per-instance kernels run above frodo_five_max (4,096): sweep them at 8,192
+    # the thread-per-instance kernels run above frodo_pair_max (9,472): sweep them at 12,288
     for tb in (32, 64, 128):
         kem.set_tuning("thread_block", tb)
-        sweep[tb] = frodo_time(8192, reps=2)[2]
+        sweep[tb] = frodo_time(12288, reps=2)[2]
     res["thread_block_ms"] = sweep
     kem.set_tuning("thread_block", min(sweep, key=sweep.get))
     # mixed batch task sizes
@@ -210,23 +212,25 @@ def _child(u: int) -> dict:
 # one lane); the stage's device time comes from the stage timer of an encaps + decaps.
 BIG = 1 << 30
 SABER_SIZES = (64, 256, 512, 1024, 2048, 4096, 8192, 16384)
-FRODO_SIZES = (64, 256, 512, 1024, 2048, 4096, 8192)
+FRODO_SIZES = (64, 256, 512, 1024, 2048, 4096, 6144, 8192)
+TC_CTAS = (0, 1, 2, 3, 4, 5, 6)  # the product's launch bound allows six
 LAYOUTS = {
-    # stage: {layout: knob values}, and the stage timer slots (encaps, decaps) it owns
+    # stage: {layout: knob values}, the stage timer slots (encaps, decaps) it owns, the form timed
     "saber_prologue": ({"warp": dict(saber_warp_max=BIG),
                         "five": dict(saber_warp_max=0, saber_five_max=BIG),
                         "pair": dict(saber_warp_max=0, saber_five_max=0, saber_pair_max=BIG),
-                        "one": dict(saber_warp_max=0, saber_five_max=0, saber_pair_max=0)}, (0,), (1,)),
+                        "one": dict(saber_warp_max=0, saber_five_max=0, saber_pair_max=0)}, (0,), (1,), "tc"),
     "saber_finish": ({"warp": dict(saber_finish_warp_max=BIG),
                       "five": dict(saber_finish_warp_max=0, saber_finish_five_max=BIG),
                       "pair": dict(saber_finish_warp_max=0, saber_finish_five_max=0, saber_pair_max=BIG),
-                      "one": dict(saber_finish_warp_max=0, saber_finish_five_max=0, saber_pair_max=0)}, (2,), ()),
-    "frodo_prologue": ({"warp": dict(frodo_warp_max=BIG),
-                        "five": dict(frodo_warp_max=0, frodo_five_max=BIG),
-                        "one": dict(frodo_warp_max=0, frodo_five_max=0)}, (0,), (1,)),
+                      "one": dict(saber_finish_warp_max=0, saber_finish_five_max=0, saber_pair_max=0)}, (2,), (), "tc"),
+    "frodo_prologue": ({"five": dict(frodo_warp_max=0, frodo_five_max=BIG),
+                        "pair": dict(frodo_warp_max=0, frodo_five_max=0, frodo_pair_max=BIG),
+                        "one": dict(frodo_warp_max=0, frodo_five_max=0, frodo_pair_max=0)}, (0,), (1,), "dp4a"),
     "frodo_ss": ({"warp": dict(frodo_ss_warp_max=BIG),
                   "five": dict(frodo_ss_warp_max=0, frodo_ss_five_max=BIG),
-                  "one": dict(frodo_ss_warp_max=0, frodo_ss_five_max=0)}, (2,), (3,)),
+                  "pair": dict(frodo_ss_warp_max=0, frodo_ss_five_max=0, frodo_pair_max=BIG),
+                  "one": dict(frodo_ss_warp_max=0, frodo_ss_five_max=0, frodo_pair_max=0)}, (2,), (3,), "dp4a"),
 }
 
 
@@ -245,40 +249,41 @@ def _lanes_sweep(eng, d, kem) -> dict:
         ss = torch.empty((n, z["ss"]), dtype=torch.uint8, device="cuda")
         return pk, sk, ec, ct, ss
 
-    def stage_ms(scheme, inputs, enc_slots, dec_slots, reps=5):
+    def stage_ms(scheme, inputs, enc_slots, dec_slots, form, reps=5):
         pk, sk, ec, ct, ss = inputs
-        eng.enc(scheme, pk, ec, d.FORM_TC, out=(ct, ss))
-        eng.dec(scheme, ct, sk, d.FORM_TC)
+        eng.enc(scheme, pk, ec, form, out=(ct, ss))
+        eng.dec(scheme, ct, sk, form)
         torch.cuda.synchronize()
         eng.profile(True)
         ts = []
         for _ in range(reps):
-            eng.enc(scheme, pk, ec, d.FORM_TC, out=(ct, ss))
+            eng.enc(scheme, pk, ec, form, out=(ct, ss))
             e = eng.stage_times()
-            eng.dec(scheme, ct, sk, d.FORM_TC)
+            eng.dec(scheme, ct, sk, form)
             x = eng.stage_times()
             ts.append(sum(e[k] for k in enc_slots) + sum(x[k] for k in dec_slots))
         eng.profile(False)
         return float(np.median(ts))
 
     out = {}
-    for stage, (layouts, es, ds) in LAYOUTS.items():
+    forms = {"tc": d.FORM_TC, "dp4a": d.FORM_DP4A}
+    for stage, (layouts, es, ds, form) in LAYOUTS.items():
         scheme = d.SABER if stage.startswith("saber") else d.FRODO976
         sweep = {}
         for n in SABER_SIZES if scheme == d.SABER else FRODO_SIZES:
             inputs = keys(scheme, n)
             for name, kv in layouts.items():
                 with kem.knobs(**kv):
-                    sweep[f"{n}/{name}"] = stage_ms(scheme, inputs, es, ds)
+                    sweep[f"{n}/{name}"] = stage_ms(scheme, inputs, es, ds, forms[form])
             del inputs
         out[f"lanes_{stage}_ms"] = sweep
     # persistent Saber tensor-core product (CTAs per SM, 0 = a CTA per instance), l=3 product stages
     psweep = {}
     for n in (1024, 4096, 16384):
         inputs = keys(d.SABER, n)
-        for per_sm in (0, 1, 2, 4, 5, 8):
+        for per_sm in TC_CTAS:
             with kem.knobs(saber_tc_ctas_per_sm=per_sm):
-                psweep[f"{n}/{per_sm}"] = stage_ms(d.SABER, inputs, (1,), (0, 2))
+                psweep[f"{n}/{per_sm}"] = stage_ms(d.SABER, inputs, (1,), (0, 2), d.FORM_TC)
         del inputs
     out["saber_tc_ctas_per_sm_ms"] = psweep
     # sponge stages of small groups as warp tasks in the persistent mixed kernel
