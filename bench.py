@@ -56,6 +56,58 @@ def dist_env():
     return env()
 
 
+# Instances up to which the tensor-core form generates all rows of A ahead (kAheadAll in csrc/frodo.cu).
+AHEAD_ALL = 1024
+
+
+def launches_per_step(tc: bool, batch: int) -> int:
+    """Kernels of an encaps and a decaps on device buffers: prologue, product and hash, and W / decode for
+    decaps; larger tensor-core batches also run the fused product for the instances not generated ahead."""
+    return 9 if tc and batch > AHEAD_ALL else 7
+
+
+def _round(x):
+    if isinstance(x, float):
+        return float(f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: _round(v) for k, v in x.items()}
+    return [_round(v) for v in x] if isinstance(x, (list, tuple)) else x
+
+
+def headline(line: dict) -> dict:
+    """The line on standard output: the headline, what explains it, and one number a section (a reader that
+    keeps only the end of the output still gets all of it).  The whole record goes to standard error."""
+    out = {k: line[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+                                "scaling", "vs_baseline", "dtype", "data", "config", "bit_exact_roundtrip",
+                                "gpu_launches", "clocks")}
+    out["roofline"] = {k: line["roofline"].get(k) for k in ("kernel", "bound", "unit", "achieved", "peak", "frac",
+                                                            "avg_launch_ms")}
+    out["stage_run"], out["stage_ms"] = line["stage_run"], line["stage_ms"]
+    if "e2e" in line:
+        out["e2e"] = {k: line["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step",
+                                                  "roundtrip_ok")}
+    if "cpu_baseline" in line:
+        out["cpu_baseline"] = {k: line["cpu_baseline"][k] for k in ("value", "unit", "cores", "kind")}
+    if "forms" in line:
+        out["forms"] = {k: line["forms"][k] for k in ("tc", "dp4a", "int32", "tc_over_dp4a",
+                                                      "product_stage_tc_over_dp4a", "product_only_tc_over_dp4a")}
+        out["frodo976aes_batch8192"] = {k: line["frodo976aes_batch8192"][k] for k in ("tc", "dp4a")}
+        out["frodo976_shared_key_batch8192"] = {k: line["frodo976_shared_key_batch8192"][k] for k in ("tc", "dp4a")}
+        out["saber_l3_batch4096"] = {k: line["saber_l3_batch4096"][k] for k in ("tc", "dp4a", "int32")}
+        out["single_request_ms"] = {k: [v["default"]["enc_ms"], v["default"]["dec_ms"]]
+                                    for k, v in line["single_request"].items()}
+        out["mixed_16384"] = {k: line["mixed_16384"][k] for k in ("tc", "tc_eager", "tc_bit_exact")}
+    if "serving" in line:
+        for f, v in line["serving"]["service"].items():
+            if isinstance(v, dict):
+                half = next(x for x in v["levels"] if x["load"] == 0.5)
+                out.setdefault("service", {})[f] = {"peak_ops_per_s": v["peak_ops_per_s"], "p50_ms_half_load": half["p50_ms"],
+                                                    "p99_ms_half_load": half["p99_ms"], "bit_exact": v["bit_exact"]}
+    if "frames_16384" in line:
+        out["frames_16384"] = {k: line["frames_16384"][k]["ops_per_s"] for k in ("frames_run", "ring_external_process")}
+    return _round(out)
+
+
 SCHEME_NAMES = {"frodo976": "FrodoKEM-976-SHAKE", "frodo976aes": "FrodoKEM-976-AES"}
 
 
@@ -134,13 +186,15 @@ def run_reference(args, world, rank):
 
 # ---------------------------------------------------------------- GPU helpers
 ONE_LANE = dict(saber_warp_max=0, saber_finish_warp_max=0, saber_five_max=0, saber_finish_five_max=0,
-                saber_pair_max=0, frodo_warp_max=0, frodo_ss_warp_max=0, frodo_five_max=0, frodo_ss_five_max=0)
+                saber_pair_max=0, frodo_warp_max=0, frodo_ss_warp_max=0, frodo_five_max=0, frodo_ss_five_max=0,
+                frodo_pair_max=0)
 
 
 def bench_single(eng, reps: int = 7) -> dict:
     """One request alone (n = 1, tc form): per-stage device times (stage timer, median of
-    `reps`) of FrodoKEM-976 and Saber l=3 encaps and decaps, the sponge stages on a warp per
-    state (the default at this size) and on one thread per state."""
+    `reps`) of FrodoKEM-976 and Saber l=3 encaps and decaps, as the call runs by default (Frodo: A's rows in the
+    prologue stage, products from tiles, encaps' hash in step with the second half of the sampling
+    stream) and with the sponge stages on one thread per state (Frodo: without tiles)."""
     import numpy as np
     import torch
 
@@ -161,12 +215,12 @@ def bench_single(eng, reps: int = 7) -> dict:
                ["prologue", "product", "finish"],
                "dec_stages": ["W / decode", "prologue", "product", "final hash"] if scheme == d.FRODO976 else
                ["inner product", "prologue", "product", "finish"]}
-        for layout, kv in (("warp_per_state", {}), ("one_lane", ONE_LANE)):
+        for layout, kv, prof in (("default", {}, True), ("one_lane", ONE_LANE, 2)):
             with K.knobs(**kv):
+                eng.profile(prof)
                 eng.enc(scheme, pk, ec, d.FORM_TC, out=(ct, ss))
                 eng.dec(scheme, ct, sk, d.FORM_TC)
                 torch.cuda.synchronize()
-                eng.profile(True)
                 es, ds = [], []
                 for _ in range(reps):
                     eng.enc(scheme, pk, ec, d.FORM_TC, out=(ct, ss))
@@ -387,9 +441,9 @@ def main():
     with sampler:
         ms, _ = timed(form, args.steps)
     clocks = sampler.summary()
-    # the stages one after the other, outside the timed region (a profiled batch of this size
-    # generates no rows ahead, so the S'A stage holds all of them)
-    _, stages = timed(form, max(3, min(args.steps, 5)), profile=True)
+    # the stages one after the other, outside the timed region and without rows generated ahead, so
+    # that the S'A stage holds all of them
+    _, stages = timed(form, max(3, min(args.steps, 5)), profile=2)
     eng.sync()
     ok = bool(torch.equal(ss, ss2))
     value = world * B * args.steps / (ms * 1e-3)
@@ -415,7 +469,7 @@ def main():
         "dtype": {d.FORM_TC: "u8xs8->s32 (tcgen05 kind::i8), u64 Keccak lanes", d.FORM_DP4A: "s16xs8->s32 (dp2a)",
                   d.FORM_INT32: "int32 multiply-add"}[form],
         "data": "synthetic (seeded SHAKE256 coins, keypairs generated on the GPU)", "config": config(args, world),
-        "bit_exact_roundtrip": ok, "gpu_launches": (9 if form == d.FORM_TC else 7) * args.steps,
+        "bit_exact_roundtrip": ok, "gpu_launches": launches_per_step(form == d.FORM_TC, B) * args.steps,
         "roofline": {
             "kernel": "sa_tc_kernel (SHAKE128 A rows in registers -> int8 tcgen05 S'A)" if form == d.FORM_TC
             else "sa_dp4a_kernel" + ("<int32>" if form == d.FORM_INT32 else ""), "bound": "int", "unit": "Gop/s",
@@ -426,6 +480,7 @@ def main():
             "keccak_per_s": B * FRODO_ROWS * FRODO_BLOCKS / (sa_avg * 1e-3),
             "keccak_peak_per_s": keccak_peak,
         },
+        "stage_run": "profiled steps after the timed ones, no rows of A ahead",
         "stage_ms": stage_ms, "stage_share_of_step": {k: sum(v.values()) / kernel_total for k, v in stage_ms.items()},
         "clocks": clocks,
     }
@@ -485,7 +540,7 @@ def main():
             for _ in range(2):
                 step(other)
             osteps = max(3, args.steps // 2)
-            oms, ostages = timed(other, osteps, profile=True)
+            oms, ostages = timed(other, osteps, profile=2)
             forms[fnames[other]] = world * B * osteps / (oms * 1e-3)
             sa_k[fnames[other]] = statistics.mean([s[1] for s in ostages["enc"]] + [s[2] for s in ostages["dec"]])
         line["forms"] = dict(forms, sa_kernel_ms=sa_k)
@@ -501,7 +556,7 @@ def main():
             for _ in range(2):
                 eng.enc(d.FRODO976AES, pk_a, ec, f, out=(ct, ss))
                 eng.dec(d.FRODO976AES, ct, sk_a, f, out=ss2)
-            eng.profile(True)
+            eng.profile(2)
             eng.enc(d.FRODO976AES, pk_a, ec, f, out=(ct, ss))
             es = eng.stage_times()
             eng.dec(d.FRODO976AES, ct, sk_a, f, out=ss2)
@@ -746,7 +801,8 @@ def main():
     peaks, src = measured_peaks()
     line["peaks_file"] = src
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps({"detail": line}), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     if pg is not None:
         pg.barrier()
         pg.destroy_process_group()

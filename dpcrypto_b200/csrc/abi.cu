@@ -255,7 +255,7 @@ int run_op(dpkem_ctx *c, int scheme, int form, int op, size_t n, const uint8_t *
     const size_t each = frodo_ahead_bytes();
     auto room = [&](size_t bytes) { return bytes / npipe > base ? (bytes / npipe - base) / each : 0; };
     size_t wish = (size_t)frodo_ahead_count((int)chunk, room(c->budget));
-    if (c->profile && wish < chunk) wish = 0;
+    if (c->profile > 1 || (c->profile && wish < chunk)) wish = 0;
     CtxMem mem(c);
     if (wish && !capturing(st)) c->arena.want(up(base + wish * each) * npipe, c->budget, mem);
     tile_cap = std::min(wish, (size_t)frodo_ahead_count((int)chunk, room(c->arena.bytes)));
@@ -827,7 +827,7 @@ int dpkem_sync(dpkem_ctx *c, void *stream) {
 int dpkem_profile(dpkem_ctx *c, int enable) {
   if (!c) return set_status(DPKEM_EINVAL);
   std::lock_guard<std::mutex> lock(c->mu);
-  c->profile = enable != 0;
+  c->profile = enable;
   c->timer_stages = 0;
   return set_status(DPKEM_OK);
 }

@@ -28,7 +28,7 @@ struct dpkem_ctx {
   uint8_t *h_stage[16] = {};      // pinned plan-table images, one per pipeline slot
   size_t h_stage_bytes[16] = {};
   cudaEvent_t stage_ev[16] = {};  // recorded after each stage's last upload
-  bool profile = false;
+  int profile = 0;  // dpkem_profile
   dpkem::StageTimer timer;
   int timer_stages = 0;
   std::mutex mu;

@@ -392,7 +392,8 @@ class Engine:
     def sync(self, stream=None):
         self._check(self._lib.dpkem_sync(self._h, stream), "sync")
 
-    def profile(self, enable: bool = True):
+    def profile(self, enable=True):
+        """Stage timing on (True), off (False), or on with every FrodoKEM batch run without operand tiles (2)."""
         self._check(self._lib.dpkem_profile(self._h, int(enable)), "profile")
 
     def stage_times(self) -> list:

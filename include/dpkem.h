@@ -205,6 +205,10 @@ int dpkem_sync(dpkem_ctx *ctx, void *stream);
  * between the kernels of its launch chain; dpkem_profile_read() waits for them and
  * returns the number of stages of the last call (its last chunk), filling stage_ms.
  * Frodo enc: prologue, S'A product, final hash; dec: W/decode, prologue, product, hash.
+ * Batches with a key per instance in the tensor-core form that generate all rows of A ahead (dpkem_ctx_create) have
+ * them in the prologue stage, and the final hash runs the second half of the sampling stream in step; larger
+ * ones run without tiles while profiled.  enable = 2: all run without, so that the product stage is the
+ * fused generation and product at every size.
  * Saber enc: prologue, product, finish; dec: inner product, prologue, product, finish. */
 int dpkem_profile(dpkem_ctx *ctx, int enable);
 int dpkem_profile_read(dpkem_ctx *ctx, float *stage_ms, int max_stages);

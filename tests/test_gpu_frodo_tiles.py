@@ -97,3 +97,20 @@ def test_profiled_batch_without_tiles(engine, oracle, scheme, n):
         eng.profile(True)
         _check(eng, oracle, scheme, case)
         assert len(eng.stage_times()) == 4 and all(t > 0 for t in eng.stage_times())
+
+
+def test_profiled_stages_without_tiles(engine, oracle):
+    """profile(2): a batch that would be generated whole runs without tiles, all of A in the product stage (with
+    tiles that stage is a pass of MMAs, a few per cent of the call)."""
+    case = _case(engine, d.FRODO976, 64)
+    kc, ec, pk, sk, ct, ss, bad, rej = case
+    with d.Engine(0) as eng:
+        share = {}
+        for mode in (True, 2):
+            eng.profile(mode)
+            _check(eng, oracle, d.FRODO976, case)
+            eng.enc(d.FRODO976, pk, ec)
+            t = eng.stage_times()
+            assert len(t) == 3
+            share[mode] = t[1] / sum(t)
+    assert share[True] < 0.15 and share[2] > 0.25, share
