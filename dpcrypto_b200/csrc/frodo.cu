@@ -349,12 +349,16 @@ cudaError_t launch_front(const FrodoBatch &b, bool halve, cudaStream_t st) {
   return launch_front_ns<STAGE, 0, false>(b, st);
 }
 
+template <int MODE, int NB>
+cudaError_t launch_product_nb(const FrodoBatch &b, cudaStream_t st) {
+  cudaError_t e;
+  if ((e = set_smem(ahead::product_kernel<MODE, NB>, ahead::PLayout::total)) != cudaSuccess) return e;
+  ahead::product_kernel<MODE, NB><<<b.ahead * (ahead::BLKS / NB), 256, ahead::PLayout::total, st>>>(b);
+  return cudaGetLastError();
+}
 template <int MODE>
 cudaError_t launch_product(const FrodoBatch &b, cudaStream_t st) {
-  cudaError_t e;
-  if ((e = set_smem(ahead::product_kernel<MODE>, ahead::PLayout::total)) != cudaSuccess) return e;
-  ahead::product_kernel<MODE><<<b.ahead * (ahead::BLKS / ahead::P_NB), 256, ahead::PLayout::total, st>>>(b);
-  return cudaGetLastError();
+  return b.ahead <= ahead::kProductFew ? launch_product_nb<MODE, 2>(b, st) : launch_product_nb<MODE, 4>(b, st);
 }
 template <bool RAW>
 cudaError_t launch_product_kp(const FrodoBatch &b, cudaStream_t st) {

@@ -4,7 +4,7 @@
 // instance) need not wait for the prologue (up to 348 dependent ones, one to a few warps'
 // worth of issue slots).  The front kernel runs both: a few blocks the sponge chains, all others
 // the rows of A, stored as operand tiles.  The product of an instance is then a pass of
-// tcgen05 MMAs over its 2.1 MB of tiles, on three CTAs.
+// tcgen05 MMAs over its 2.1 MB of tiles, on three CTAs (few instances: six).
 //
 //   front    blocks [0, chain): the prologue's sponges; [chain, chain + absorb): decaps'
 //            ciphertext pre-absorb; the rest: 256 rows of A each, a row per thread
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(32) kp_seed_kernel(FrodoBatch b) {
 }
 
 // ---------------------------------------------------------------- product S'A
-// CTA (256 threads) = one instance, P_NB column blocks from b0 on.  Warp 0 lane 0 moves the tiles
+// CTA (256 threads) = one instance, column blocks [b0, b0 + NB).  Warp 0 lane 0 moves the tiles
 // (one bulk copy each) through an NST-stage mbarrier ring, warp 1 lane 0 issues the MMAs (per
 // 32 rows: bytes 0..127 and 128..167 of the block, N = 8), the CTA of the last block also forms
 // V = S'B on warps 2..7 meanwhile.  All eight warps read the accumulators back.
@@ -270,11 +270,12 @@ __global__ void __launch_bounds__(32) kp_seed_kernel(FrodoBatch b) {
 // the errors.  PM_ENC: ciphertext.  PM_DEC: compare, an OR into the fail word.
 enum PMode : int { PM_RAW = 0, PM_ENC = 1, PM_DEC = 2 };
 constexpr int P_NST = 4;
-// Column blocks of a CTA: four read S' three times an instance; narrower CTAs for few instances gain nothing.  us, 1 / 2 / 4
-// blocks, encaps: n = 1 745 / 744 / 744, 32 783 / 781 / 778, 128 846 / 842 / 833, 1,024 3,786 / 3,722 / 3,700; decaps at
-// 1,024 3,618 / 3,536 / 3,503.
-constexpr int P_NB = 4;
-constexpr uint32_t P_TMEM = 64;
+// Column blocks of a CTA: four read S' three times an instance; up to kProductFew instances two, whose MMAs are half as
+// many one after the other.  us, 1 / 2 / 4 blocks, decaps: n = 1 502 / 501 / 504, 8 528 / 527 / 530, 24 534 / 532 / 534, 32
+// 554 / 547 / 548, 128 617 / 609 / 600, 1,024 3,618 / 3,536 / 3,503; encaps: 1 745 / 744 / 744, 32 783 / 781 / 778, 1,024 3,786 / 3,722 /
+// 3,700.
+constexpr int kProductFew = 24;
+__host__ __device__ constexpr uint32_t product_cols(int nb) { return nb <= 2 ? 32 : 64; }  // TMEM columns
 
 struct PLayout {
   static constexpr int sp = 0;                                   // S' operand, 62 * 128
@@ -286,14 +287,14 @@ struct PLayout {
   static constexpr int total = red + 3 * 64 * 4;
 };
 
-template <int MODE>
+template <int MODE, int NB>
 __global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b) {
   using L = PLayout;
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int op = MODE == PM_DEC ? OP_DEC : OP_ENC;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int parts = BLKS / P_NB, nst = P_NB * TILES;
-  const int inst = blockIdx.x / parts, b0 = (blockIdx.x % parts) * P_NB, b1 = b0 + P_NB;
+  constexpr int parts = BLKS / NB, nst = NB * TILES;
+  const int inst = blockIdx.x / parts, b0 = (blockIdx.x % parts) * NB, b1 = b0 + NB;
   const Inst v = inst_of(b, inst, op);
   const uint8_t *tiles = b.atile + (size_t)inst * A_BYTES;
   uint8_t *sp = smem + L::sp;
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b) {
   uint32_t(*red)[64] = reinterpret_cast<uint32_t(*)[64]>(smem + L::red);
   const uint16_t *rw = v.rw;
   if (warp == 0) {
-    tmem_alloc(tslot, P_TMEM);
+    tmem_alloc(tslot, product_cols(NB));
     tmem_relinquish();
   }
   if (tid == 32) {
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(256, 2) product_kernel(FrodoBatch b) {
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tbase, P_TMEM);
+    tmem_dealloc(tbase, product_cols(NB));
   }
 }
 

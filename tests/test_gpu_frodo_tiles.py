@@ -74,6 +74,12 @@ def test_reserved_arena(engine, oracle, scheme, n, mib, tiles):
         _check(eng, oracle, scheme, case)
 
 
+@pytest.mark.parametrize("scheme,n", [(d.FRODO976, 24), (d.FRODO976, 25), (d.FRODO976AES, 24)])
+def test_product_blocks(engine, oracle, scheme, n):
+    """Two column blocks a product CTA up to 24 instances, four above."""
+    _check(engine, oracle, scheme, _case(engine, scheme, n))
+
+
 @pytest.mark.parametrize("scheme", [d.FRODO976, d.FRODO976AES])
 def test_budget_without_tiles(engine, oracle, scheme):
     """A budget of 4 MiB: half of it is scratch, chunks of 66 and 34, no room for tiles; host buffers too."""
