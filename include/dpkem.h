@@ -271,9 +271,10 @@ int dpkem_saber_enc_batch_static(int scheme, int form, size_t n, const uint8_t *
  * "mixed_thread_task" (instances per thread-level task in mixed batches), "pipe_chunks"
  * (chunks, one stream each, of a pipelined host-buffer batch, <= 16), "pipe_priority" (0/1:
  * chunk streams with descending priorities, so earlier chunks finish first),
- * "saber_pair_max" (Keccak lanes per state in the Saber prologue: batches of up to this many
- * instances run GenMatrix on two lanes per state, larger ones on one; 0 = never).  Chosen by
- * dpcrypto_b200/autotune.py and stored in dpcrypto_b200/tuning.json. */
+ * "saber_pair_max" (Saber batches of up to this many instances run their sponges on two Keccak lanes per state,
+ * larger ones on one; 0 = never), "saber_five_max", "frodo_pair_max" and the like (lanes per state of the other
+ * stages).  Chosen by dpcrypto_b200/autotune.py, stored in dpcrypto_b200/tuning.json and compiled in as the
+ * defaults. */
 int dpkem_set_tuning(const char *key, int value);
 /* Current value of a knob (DPKEM_EINVAL for an unknown key). */
 int dpkem_get_tuning(const char *key, int *value);
