@@ -156,7 +156,9 @@ int dpkem_mixed_graph_destroy(dpkem_graph *g);
  * The kernel ends after idle_ms without work and is relaunched by the next submit, poll or
  * drain.  Every device wait is bounded; an expired one makes poll / drain / close return
  * DPKEM_ETIMEOUT.  While a service is open its launch holds the CTA slots it was given
- * (dpkem_ctx_set_max_ctas caps them): other kernels on the device share what is left.
+ * (dpkem_ctx_set_max_ctas caps them): other kernels on the device share what is left.  FrodoKEM batches
+ * enqueued while a service is open run without operand tiles, in kernels that fit beside one of its CTAs; one that
+ * was enqueued or captured before may wait for the launch's end.
  * No counterpart in the reference (FrodoKEM976-GPU/main.cu:13-34, SABER-GPU/main.cu:12-38
  * run one fixed batch per program). */
 typedef struct dpkem_service dpkem_service;
